@@ -887,35 +887,6 @@ __global__ void residual_sketch_kernel(const T* __restrict__ x, const float* __r
     }
 }
 
-// compute_logit_bias (src/cache/tq.rs:185-253): bias[h, i, t] = (sum_d rq[h, i, d] * (+-1)) * c_t with
-// c_t = norm_t * sqrt(pi/2) / sqrt(D).  One thread per token, the group's projected queries in shared memory.
-// rq: [hq, q_len, D]; signs: [hkv, stride, D/8]; norms: [hkv, stride]; bias: [hq, q_len, kv_len] of type OT.
-template <typename OT>
-__global__ void logit_bias_kernel(const float* __restrict__ rq, const uint8_t* __restrict__ signs,
-                                  const uint16_t* __restrict__ norms, OT* __restrict__ bias, int hq, int hkv, int q_len,
-                                  int D, int kv_len, int kv_stride, float scale_factor) {
-    extern __shared__ float s_rq[];   // [g * q_len][D]
-    const int kvh = blockIdx.y, g = hq / hkv;
-    const int rows = g * q_len;
-    for (int i = threadIdx.x; i < rows * D; i += blockDim.x) s_rq[i] = rq[(size_t)kvh * rows * D + i];
-    __syncthreads();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= kv_len) return;
-    const size_t row = (size_t)kvh * kv_stride + t;
-    const uint32_t* sw = reinterpret_cast<const uint32_t*>(signs + row * (D / 8));
-    const float c = f16_bits_to_f32(norms[row]) * scale_factor;
-    for (int r = 0; r < rows; ++r) {
-        float acc = 0.0f;
-        for (int w = 0; w < D / 32; ++w) {
-            const uint32_t bits = sw[w];
-#pragma unroll 8
-            for (int b = 0; b < 32; ++b) acc = fmaf(s_rq[r * D + w * 32 + b], ((bits >> b) & 1u) ? 1.0f : -1.0f, acc);
-        }
-        const int head = kvh * g + r / q_len, qi = r % q_len;
-        bias[((size_t)head * q_len + qi) * kv_len + t] = from_f32<OT>(acc * c);
-    }
-}
-
 size_t quant_smem(int dim, int pb, int warps, bool qjl) {
     const int W = dim / 32;
     size_t per_warp = sizeof(float) * kTile * (dim + 1) + dim + (size_t)kTile * pb;
@@ -1244,38 +1215,6 @@ int tqb_residual_sketch(int32_t dim, const uint32_t* rbits, const void* original
     else if (dtype == TQB_F16) TQB_SKETCH(__half);
     else TQB_SKETCH(__nv_bfloat16);
 #undef TQB_SKETCH
-    return check_launch(s);
-}
-
-int tqb_qjl_logit_bias(int32_t head_dim, const float* rq, const uint8_t* signs, const uint16_t* norms, void* bias,
-                       int32_t bias_dtype, int32_t num_q_heads, int32_t num_kv_heads, int32_t q_len, int32_t kv_len,
-                       int32_t kv_stride, tqb_stream_t stream) {
-    TQB_NVTX_RANGE();
-    if (head_dim <= 0 || head_dim % 32 != 0) return TQB_ERR_INVALID_DIMENSION;
-    if (num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0 || q_len <= 0) return TQB_ERR_INVALID_ARGUMENT;
-    if (kv_len < 0 || kv_len > kv_stride) return TQB_ERR_RANGE_OUT_OF_BOUNDS;
-    if (kv_len == 0) return TQB_OK;
-    if (!rq || !signs || !norms || !bias) return TQB_ERR_NULL_POINTER;
-    if ((uintptr_t)signs % 4) return TQB_ERR_MISALIGNED;
-    const int g = num_q_heads / num_kv_heads;
-    const size_t smem = sizeof(float) * (size_t)g * q_len * head_dim;
-    if (smem > 200 * 1024) return TQB_ERR_TOO_LARGE;
-    // src/cache/tq.rs:215-216: sqrt(pi/2) as f32 divided by sqrt(head_dim) in f32
-    const float scale_factor = (float)sqrt(1.5707963267948966) / sqrtf((float)head_dim);
-    cudaStream_t s = as_stream(stream);
-    dim3 grid((kv_len + 127) / 128, num_kv_heads);
-#define TQB_BIAS(OT)                                                                                                   \
-    do {                                                                                                               \
-        cudaError_t e = cudaFuncSetAttribute(logit_bias_kernel<OT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        if (e != cudaSuccess) { set_cuda_error(e); return TQB_ERR_CUDA; }                                              \
-        logit_bias_kernel<OT><<<grid, 128, smem, s>>>(rq, signs, norms, (OT*)bias, num_q_heads, num_kv_heads, q_len,   \
-                                                      head_dim, kv_len, kv_stride, scale_factor);                      \
-    } while (0)
-    if (bias_dtype == TQB_F32) TQB_BIAS(float);
-    else if (bias_dtype == TQB_F16) TQB_BIAS(__half);
-    else if (bias_dtype == TQB_BF16) TQB_BIAS(__nv_bfloat16);
-    else return TQB_ERR_INVALID_ARGUMENT;
-#undef TQB_BIAS
     return check_launch(s);
 }
 
