@@ -403,6 +403,8 @@ int tqb_pqo_cache_dequantize_full(tqb_pqo_cache *c, int32_t layer, void *k_out, 
                                   int32_t host_buffers, tqb_stream_t stream);
 int64_t tqb_pqo_cache_seq_len(const tqb_pqo_cache *c, int32_t layer);
 int64_t tqb_pqo_cache_capacity(const tqb_pqo_cache *c, int32_t layer);
+/* Drops every layer's rows.  Device memory: up to 512 MB of the freed blocks stay with the cache for its next rows and go
+ * with tqb_pqo_cache_destroy; the rest is freed. */
 int tqb_pqo_cache_reset(tqb_pqo_cache *c);
 /* enabled != 0: the decode launches of this cache (tqb_pqo_cache_decode with device buffers, tqb_pqo_cache_attend_partial,
  * tqb_pqo_cache_attend_push) are made with TQB_DECODE_OVERLAP whenever the layer differs from the layer of the

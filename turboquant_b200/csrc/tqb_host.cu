@@ -50,6 +50,68 @@ struct DevBuf {
     }
 };
 
+// Blocks of device memory that a cache object gives up (reset, growth) and takes again: cudaMalloc and cudaFree cost
+// about 80 us each and cudaFree waits for the whole device, so a request of 16 steps on 28 layers spent 18 of its 20 ms
+// in them.  The pool belongs to one cache object, keeps at most kKeepBytes and is given back with the object or when
+// an allocation fails.  Every block in it is idle: its owner has synchronised the device before it was put here.
+struct BlockPool {
+    static constexpr size_t kKeepBytes = 512u << 20;
+    struct Block {
+        void* p;
+        size_t bytes;
+    };
+    std::vector<Block> idle;
+    size_t held = 0;
+
+    // The smallest idle block that fits, unless it is more than twice as large; else a new one.  `use_idle` = false while
+    // the stream is being captured: whatever cudaMalloc answers there is the answer.
+    cudaError_t take(size_t need, bool use_idle, void** p, size_t* bytes) {
+        size_t best = idle.size();
+        for (size_t i = 0; use_idle && i < idle.size(); ++i)
+            if (idle[i].bytes >= need && idle[i].bytes / 2 <= need && (best == idle.size() || idle[i].bytes < idle[best].bytes)) best = i;
+        if (best != idle.size()) {
+            *p = idle[best].p;
+            *bytes = idle[best].bytes;
+            held -= idle[best].bytes;
+            idle.erase(idle.begin() + best);
+            return cudaSuccess;
+        }
+        cudaError_t e = cudaMalloc(p, need);
+        if (e == cudaErrorMemoryAllocation && !idle.empty()) {
+            cudaGetLastError();
+            trim();
+            e = cudaMalloc(p, need);
+        }
+        *bytes = need;
+        return e;
+    }
+    void put(void* p, size_t bytes) {
+        if (!p) return;
+        if (held + bytes > kKeepBytes) {
+            cudaFree(p);
+            return;
+        }
+        idle.push_back(Block{p, bytes});
+        held += bytes;
+    }
+    void trim() {
+        for (auto& b : idle) cudaFree(b.p);
+        idle.clear();
+        held = 0;
+    }
+};
+
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {   // the legacy stream while another one is being captured
+        cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
+size_t align256(size_t n) { return (n + 255) / 256 * 256; }
+
 }  // namespace
 
 // ---------------------------------------------------------------------------------------
@@ -82,8 +144,11 @@ struct tqb_pqo_cache {
         uint16_t *ks = nullptr, *vs = nullptr;
         int64_t cap = 0, len = 0;
         bool active = false;
+        void* block = nullptr;   // one allocation: K indices, V indices, K scales, V scales, each 256-byte aligned
+        size_t block_bytes = 0;
     };
     std::vector<Layer> layers;
+    BlockPool pool;
     DevBuf stage_k, stage_v, stage_q, stage_out, scratch;
     // tqb_pqo_cache_set_overlap: decode launches of different layers may start before their predecessor has finished
     bool overlap = false;
@@ -127,11 +192,9 @@ struct tqb_pqo_cache {
         copy_stream = down_stream = nullptr;
     }
 
+    // (nothing queued uses the layer any more)
     void free_layer(Layer& l) {
-        if (l.ki) cudaFree(l.ki);
-        if (l.vi) cudaFree(l.vi);
-        if (l.ks) cudaFree(l.ks);
-        if (l.vs) cudaFree(l.vs);
+        pool.put(l.block, l.block_bytes);
         l = Layer{};
     }
 
@@ -148,19 +211,17 @@ struct tqb_pqo_cache {
         nl.active = l.active;
         const size_t ib = (size_t)heads * new_cap * packed_dim;
         const size_t sb = (size_t)heads * new_cap * nblk * sizeof(uint16_t);
+        const size_t ia = align256(ib), sa = align256(sb);
         cudaError_t e;
-        if ((e = cudaMalloc((void**)&nl.ki, ib)) != cudaSuccess || (e = cudaMalloc((void**)&nl.vi, ib)) != cudaSuccess ||
-            (e = cudaMalloc((void**)&nl.ks, sb)) != cudaSuccess || (e = cudaMalloc((void**)&nl.vs, sb)) != cudaSuccess) {
-            free_layer(nl);
-            return cuda_fail(e);
-        }
+        if ((e = pool.take(2 * (ia + sa), !capturing(s), &nl.block, &nl.block_bytes)) != cudaSuccess) return cuda_fail(e);
+        nl.ki = (uint8_t*)nl.block;
+        nl.vi = nl.ki + ia;
+        nl.ks = (uint16_t*)(nl.vi + ia);
+        nl.vs = (uint16_t*)(nl.vi + ia + sa);
         // on any failure from here on the new buffers are released and the layer is left as it was
         auto fill = [&]() -> cudaError_t {
             cudaError_t r;
-            if ((r = cudaMemsetAsync(nl.ki, 0, ib, s)) != cudaSuccess) return r;
-            if ((r = cudaMemsetAsync(nl.vi, 0, ib, s)) != cudaSuccess) return r;
-            if ((r = cudaMemsetAsync(nl.ks, 0, sb, s)) != cudaSuccess) return r;
-            if ((r = cudaMemsetAsync(nl.vs, 0, sb, s)) != cudaSuccess) return r;
+            if ((r = cudaMemsetAsync(nl.block, 0, 2 * (ia + sa), s)) != cudaSuccess) return r;
             if (l.len > 0) {
                 const size_t iw = (size_t)l.len * packed_dim, sw = (size_t)l.len * nblk * 2;
                 if ((r = cudaMemcpy2DAsync(nl.ki, (size_t)new_cap * packed_dim, l.ki, (size_t)l.cap * packed_dim, iw, heads,
@@ -172,12 +233,12 @@ struct tqb_pqo_cache {
                 if ((r = cudaMemcpy2DAsync(nl.vs, (size_t)new_cap * nblk * 2, l.vs, (size_t)l.cap * nblk * 2, sw, heads,
                                            cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return r;
             }
-            // the old buffers may still be read by queued work, and the copies above must have left them
-            return l.ki ? cudaStreamSynchronize(s) : cudaSuccess;
+            // the old buffers may still be read by work queued on any stream, and the copies above must have left them
+            return l.ki ? cudaDeviceSynchronize() : cudaSuccess;
         };
         if ((e = fill()) != cudaSuccess) {
-            cudaStreamSynchronize(s);   // nothing queued may still write the buffers that are released next
-            free_layer(nl);
+            cudaDeviceSynchronize();   // nothing queued may still write the buffers that are released next
+            cudaFree(nl.block);
             return cuda_fail(e);
         }
         if (l.ki) free_layer(l);
@@ -356,7 +417,8 @@ int tqb_pqo_cache_create(const tqb_cache_config* cfg, tqb_pqo_cache** out) {
 
 void tqb_pqo_cache_destroy(tqb_pqo_cache* c) {
     if (!c) return;
-    for (auto& l : c->layers) c->free_layer(l);
+    for (auto& l : c->layers) cudaFree(l.block);   // waits for the device
+    c->pool.trim();
     c->stage_k.release(); c->stage_v.release(); c->stage_q.release(); c->stage_out.release(); c->scratch.release();
     c->destroy_pipeline();
     delete c;
@@ -531,7 +593,7 @@ int tqb_pqo_cache_set_overlap(tqb_pqo_cache* c, int32_t enabled) {
     return TQB_OK;
 }
 
-// CompressedStorage::reset (src/cache/storage.rs:175-185): drops the buffers.
+// CompressedStorage::reset (src/cache/storage.rs:175-185): drops the buffers (the cache's block pool keeps a bounded part).
 int tqb_pqo_cache_reset(tqb_pqo_cache* c) {
     if (!c) return TQB_ERR_NULL_POINTER;
     TQB_CUDA(cudaDeviceSynchronize());
@@ -887,6 +949,7 @@ struct tqb_tq_cache {
         uint8_t* signs = nullptr;
         uint16_t* norms = nullptr;
         int64_t cap = 0;
+        size_t block_bytes = 0;   // one allocation that starts at `signs`
     };
     std::vector<Q> qjl;
     uint32_t* rbits = nullptr;
@@ -895,8 +958,7 @@ struct tqb_tq_cache {
     int sb() const { return base->cfg.head_dim / 8; }
 
     void free_q(Q& q) {
-        if (q.signs) cudaFree(q.signs);
-        if (q.norms) cudaFree(q.norms);
+        base->pool.put(q.signs, q.block_bytes);
         q = Q{};
     }
 
@@ -908,27 +970,24 @@ struct tqb_tq_cache {
         Q n;
         n.cap = new_cap;
         const int heads = base->heads;
+        const size_t sa = align256((size_t)heads * new_cap * sb()), bytes = sa + align256((size_t)heads * new_cap * 2);
         cudaError_t e;
-        if ((e = cudaMalloc((void**)&n.signs, (size_t)heads * new_cap * sb())) != cudaSuccess ||
-            (e = cudaMalloc((void**)&n.norms, (size_t)heads * new_cap * 2)) != cudaSuccess) {
-            free_q(n);
-            return cuda_fail(e);
-        }
+        if ((e = base->pool.take(bytes, !capturing(s), (void**)&n.signs, &n.block_bytes)) != cudaSuccess) return cuda_fail(e);
+        n.norms = (uint16_t*)(n.signs + sa);
         auto fill = [&]() -> cudaError_t {
             cudaError_t r;
-            if ((r = cudaMemsetAsync(n.signs, 0, (size_t)heads * new_cap * sb(), s)) != cudaSuccess) return r;
-            if ((r = cudaMemsetAsync(n.norms, 0, (size_t)heads * new_cap * 2, s)) != cudaSuccess) return r;
+            if ((r = cudaMemsetAsync(n.signs, 0, bytes, s)) != cudaSuccess) return r;
             if (old_len > 0 && q.signs) {
                 if ((r = cudaMemcpy2DAsync(n.signs, (size_t)new_cap * sb(), q.signs, (size_t)q.cap * sb(), (size_t)old_len * sb(),
                                            heads, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return r;
                 if ((r = cudaMemcpy2DAsync(n.norms, (size_t)new_cap * 2, q.norms, (size_t)q.cap * 2, (size_t)old_len * 2, heads,
                                            cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return r;
             }
-            return q.signs ? cudaStreamSynchronize(s) : cudaSuccess;
+            return q.signs ? cudaDeviceSynchronize() : cudaSuccess;
         };
         if ((e = fill()) != cudaSuccess) {
-            cudaStreamSynchronize(s);
-            free_q(n);
+            cudaDeviceSynchronize();
+            cudaFree(n.signs);
             return cuda_fail(e);
         }
         if (q.signs) free_q(q);
@@ -1006,7 +1065,7 @@ int tqb_tq_cache_create(const tqb_cache_config* cfg, tqb_tq_cache** out) {
 
 void tqb_tq_cache_destroy(tqb_tq_cache* c) {
     if (!c) return;
-    for (auto& q : c->qjl) c->free_q(q);
+    for (auto& q : c->qjl) cudaFree(q.signs);
     if (c->rbits) cudaFree(c->rbits);
     c->deq.release(); c->qf32.release(); c->rq.release();
     tqb_pqo_cache_destroy(c->base);
