@@ -1,10 +1,11 @@
-"""GPU kernels of the sign sketch at the edges of their tiles: the logit bias on the tensor cores."""
+"""GPU kernels of the sign sketch at the edges of their tiles and on awkward vectors."""
 import ctypes
 
 import numpy as np
 import pytest
 import torch
 
+import turboquant_b200 as tq
 from turboquant_b200._lib import lib
 
 pytestmark = pytest.mark.gpu
@@ -33,3 +34,61 @@ def test_logit_bias_at_tile_edges(dim, group, q_len, kv_len):
     # the running magnitude per addition, and the final scaling twice
     bound = (3 * dim + 4) * 2.0 ** -23 * rq.double().abs().sum(-1)[..., None] * c[:, None] + 1e-30
     assert bool(((bias.double() - want).abs() <= bound).all())
+
+
+def _stream():
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _awkward(n, dim, seed):
+    """Vectors with sums that tie or nearly cancel, all-zero ones, denormal and huge ones, infinities and NaN among ordinary ones."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn((n, dim), generator=g, device="cuda")
+    kind = torch.arange(n, device="cuda") % 9
+    x[kind == 1] = 0.0
+    x[kind == 2] = x[kind == 2].sign()                        # +-1: many sums are exactly zero in some order
+    x[kind == 3] = x[kind == 3] * 1e-30
+    x[kind == 4] = x[kind == 4] * 1e30
+    x[kind == 5] = torch.round(x[kind == 5] * 4)              # small integers
+    if n > 60:
+        x[7, 3], x[16, dim - 1], x[25, 0] = float("inf"), float("nan"), float("-inf")
+    return x
+
+
+@pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("dim,n", [(32, 16), (32, 1000), (64, 33), (64, 700), (128, 17), (128, 31), (128, 2500), (256, 20), (256, 900)])
+def test_qjl_quantize_batches_equal_single_vectors(dim, n, bits):
+    # the bytes of a batch on the tensor cores are those of the sequential sums, which calls of a few vectors take
+    cfg = tq.TurboQuantConfig(bits, dim).with_seed(7)
+    x = _awkward(n, dim, dim + n)
+    got = tq.qjl_quantize_batch(cfg, x, 5)
+    pieces = [tq.qjl_quantize_batch(cfg, x[a:a + 15], 5) for a in range(0, n, 15)]
+    for i, name in enumerate(("packed", "scales", "signs", "rnorms")):
+        assert torch.equal(got[i], torch.cat([p[i] for p in pieces])), name
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dim", [32, 64, 128, 256])
+def test_residual_sketch_tiles_equal_single_vectors(dim, dtype):
+    n, rpg, gs, off = 2048 + 37, 139, 200, 11                 # 15 groups of 139 rows at rows 11.. of 200
+    x = _awkward(n, dim, dim).to(dtype)
+    xhat = (x.float() * 0.9 + 0.02).nan_to_num(1.0, 2.0, -2.0)
+    rb = tq.api.rademacher_bits(dim, 9, x.device)
+    code = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}[dtype]
+    outs = []
+    for step in (n, rpg):                                     # one call on the tensor cores; one per group, sequential sums
+        signs = torch.zeros((15 * gs, dim // 8), dtype=torch.uint8, device="cuda")
+        norms = torch.zeros((15 * gs,), dtype=torch.int16, device="cuda")
+        for a in range(0, n, step):
+            assert lib.tqb_residual_sketch(dim, _p(rb), _p(x[a:]), code, _p(xhat[a:]), step, _p(signs[a // rpg * gs:]), _p(norms[a // rpg * gs:]),
+                                           rpg, gs, off, _stream()) == 0
+        outs.append((signs, norms))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("dim", [32, 64, 128, 256])
+def test_projections_of_many_queries_equal_single_ones(dim):
+    q = _awkward(2048 + 13, dim, 3)
+    many = tq.query_projections(q, dim, 21)
+    few = torch.cat([tq.query_projections(q[a:a + 100], dim, 21) for a in range(0, len(q), 100)])
+    assert torch.equal(many.nan_to_num(7.0, 8.0, -8.0), few.nan_to_num(7.0, 8.0, -8.0))

@@ -14,6 +14,7 @@
 
 #include "tqb_common.cuh"
 #include "tqb_pqo_quant.cuh"
+#include "tqb_sketch.cuh"
 #include <type_traits>
 
 namespace tqb {
@@ -967,6 +968,11 @@ int grid_warps(long long n, int warps_per_block) {
     return (int)g;
 }
 
+// From these batch sizes on the kernels of tqb_sketch.cu take over.  Quantize with sketch: two launches of about 19 us
+// against 8 us + 2.1 us a vector (128 dims: 16 vectors 19 against 41 us, 8 vectors 25 us sequentially).  Residual sketch and projections: below
+// 2,048 vectors one vector or query per warp fills the chip and takes 6 to 9 us; at 4,096 the tiles are ahead.
+constexpr long long kSketchMin = 16, kResidualTileMin = 2048, kProjTileMin = 2048;
+
 float host_inv_sqrt(int dim) { return 1.0f / sqrtf((float)dim); }  // rotation.rs:36
 
 }  // namespace
@@ -1022,7 +1028,13 @@ int tqb_qjl_quantize_batch(const tqb_config* cfg, const uint32_t* rbits, const f
     a.x = x; a.n = n; a.packed = packed; a.scales = scales; a.signs = signs; a.rnorms = rnorms; a.rbits = rbits;
     a.bits = polar.bits; a.dim = polar.dim; a.pb = (int)tqb_packed_bytes(polar.bits, polar.dim);
     a.seed = cfg->rotation_seed; a.inv_sqrt_d = host_inv_sqrt(cfg->dim);
-    return dispatch_quant<true>(a, cb, as_stream(stream));
+    cudaStream_t s = as_stream(stream);
+    if (n >= kSketchMin && polar.bits <= 3 && ((uintptr_t)x % 16) == 0 && cell_table_fits(cb, polar.bits)) {
+        st = dispatch_quant<false>(a, cb, s);
+        if (st != TQB_OK) return st;
+        return launch_whole_sketch(a.dim, a.bits, x, packed, scales, n, rbits, signs, rnorms, cb, (int)(a.seed & 1ULL), a.inv_sqrt_d, s);
+    }
+    return dispatch_quant<true>(a, cb, s);
 }
 
 static int dequant_common(const tqb_config* cfg, const uint8_t* packed, const uint16_t* scales, int64_t n, float* out,
@@ -1073,6 +1085,7 @@ int tqb_qjl_query_projections(int32_t dim, const uint32_t* rbits, const float* q
     if (nq == 0) return TQB_OK;
     if (!rbits || !q || !rq) return TQB_ERR_NULL_POINTER;
     cudaStream_t s = as_stream(stream);
+    if (nq >= kProjTileMin) return launch_projections_tile(dim, q, TQB_F32, nq, rbits, rq, host_inv_sqrt(dim), s);
     const int W = dim / 32, warps = 4;
     const size_t smem = sizeof(uint32_t) * dim * (W + 1) + sizeof(float) * warps * dim;
     const int grid = grid_warps(nq, warps);
@@ -1192,6 +1205,9 @@ int tqb_residual_sketch(int32_t dim, const uint32_t* rbits, const void* original
     if ((uintptr_t)signs % 4) return TQB_ERR_MISALIGNED;
     if (dtype != TQB_F32 && dtype != TQB_F16 && dtype != TQB_BF16) return TQB_ERR_INVALID_ARGUMENT;
     cudaStream_t s = as_stream(stream);
+    if (n >= kResidualTileMin && ((uintptr_t)original % 16) == 0 && ((uintptr_t)dequantized % 16) == 0)
+        return launch_residual_sketch(dim, original, dtype, dequantized, n, rbits, signs, norms, rows_per_group, out_group_stride,
+                                      out_row_offset, host_inv_sqrt(dim), s);
     const int W = dim / 32, warps = dim >= 256 ? 2 : 4;
     // vectors per warp tile: enough tiles for ~16 warps on every SM before a warp takes a second vector
     long long vt = (n + 148 * 16 - 1) / (148 * 16);
