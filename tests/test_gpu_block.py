@@ -154,3 +154,31 @@ def test_quantize_dequantize_idempotence_at_bulk_size():
         rows = torch.arange(0, n, 997, device="cuda")
         op, os_ = o.block_quantize(bits, 128, 0, -1, x[rows].float().cpu().numpy(), nthreads=8)
         assert np.array_equal(idx[rows].cpu().numpy(), op) and np.array_equal(u16(sc[rows]), os_)
+
+
+def _rows_at(shift, n, width, dtype):
+    """[n, width] bytes whose start lies `shift` bytes behind a 16-byte boundary."""
+    return torch.zeros(n * width + 16, dtype=torch.uint8, device="cuda")[shift:shift + n * width].view(n, width).view(dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("bits,ob", [(3, -1), (3, 0), (4, -1), (4, 0)])
+@pytest.mark.parametrize("head_dim,n,rpg", [(32, 1, 0), (32, 33, 0), (64, 300, 7), (96, 21, 3), (128, 65, 13), (160, 130, 0), (256, 1000, 250)])
+def test_one_codebook_kernels_equal_the_general_ones(bits, ob, dtype, head_dim, n, rpg):
+    # code arrays that start off a 16-byte boundary take the general kernels (four lanes a block)
+    x = (torch.randn((n, head_dim), generator=torch.Generator().manual_seed(n + bits)) * 3).cuda().to(dtype)
+    x[::5] *= 1e-3
+    x[3::7] = 0
+    gs, off = (rpg + 5, 2) if rpg else (0, 0)
+    rows = -(-n // rpg) * gs + off if rpg else n
+    pd, nb, code = head_dim * bits // 8, head_dim // 32, {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}[dtype]
+    got = []
+    for shift in (0, 4):
+        idx, sc = _rows_at(shift, rows, pd, torch.uint8), torch.zeros((rows, nb), dtype=torch.int16, device="cuda")
+        tq.block_quantize(x, bits, outlier_blocks=ob, out=(idx, sc), rows_per_group=rpg, group_stride=gs, row_offset=off)
+        out = torch.empty_like(x)
+        s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert lib.tqb_block_dequantize(bits, head_dim, 0, ob, ptr(idx), ptr(sc), n, rpg, gs, off, ptr(out), code, s) == 0
+        got.append((idx.clone(), sc, out))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

@@ -4,6 +4,7 @@
 // src/cache/cuda/kernels/tq_quant_kernel.cu:216-259; results are bit-identical to the general kernel.
 #pragma once
 #include "tqb_common.cuh"
+#include "tqb_f32x2.cuh"
 
 namespace tqb {
 
@@ -62,99 +63,153 @@ __device__ __forceinline__ void butterfly32_regs(float (&v)[32]) {
 constexpr uint32_t kSignMask = 0xB1A6D4B2u;   // bit j set <=> sign j is -1 (precomputed/rotation.rs:16-20)
 
 
-// Cell table for the 3-bit boundary search: cell c = round(t * kCellScale + kCellHalf); the 256 cells are far narrower
-// than the gap between two boundaries, so a cell (widened by kCellSlop on both sides to absorb the rounding
-// of the cell index) holds at most one boundary:  code = below + (t > bnd), exactly the count of
-// boundaries below t.  .x = that boundary (FLT_MAX when the cell has none), .y = bit pattern of the number
-// of boundaries under the cell.  |t| <= outer centroid (2.1520 for the 3-bit table) < 2.2 by construction
-// of the MaxNorm scale, so the index never leaves the table.
-constexpr float kCellScale = 58.0f;
-constexpr float kCellHalf = 128.0f;   // an integer, so that kCellHalf + 1.5 * 2^23 is exact
+// Cell table for the boundary search of the small codebooks: cell k >> 8 of k = round(t * kCellScale + kCellHalf), 32
+// cells of 0.138 - narrower than any gap between two boundaries (0.49), so a cell (widened by kCellSlop on both sides to
+// absorb the rounding of k) holds at most one boundary:  code = below + (t > bnd), exactly the count of
+// boundaries below t.  .x = that boundary (3e38 when the cell has none), .y = the number of boundaries under the cell.
+// Stored [cell][lane]: the 32 look-ups of a warp instruction touch 32 different bank pairs (256 unreplicated cells met
+// ~6 wavefronts a look-up).  |t| <= outer centroid (2.1573) < 2.2 by construction of the MaxNorm scale, so k stays inside.
+constexpr int kCells = 32;
+constexpr float kCellScale = 1856.0f;
+constexpr float kCellHalf = 4096.0f;   // an integer, so that kCellHalf + 1.5 * 2^23 is exact
 constexpr float kCellSlop = 1e-3f;
 __device__ __forceinline__ void build_cell_table(const Codebook& cb, int n_bnd, float2* lut, int tid, int nthreads) {
-    for (int c = tid; c < 256; c += nthreads) {
-        const float lo = ((float)c - 0.5f - kCellHalf) / kCellScale - kCellSlop;
-        const float hi = ((float)c + 0.5f - kCellHalf) / kCellScale + kCellSlop;
+    for (int i = tid; i < kCells * 32; i += nthreads) {
+        const int c = i >> 5;
+        const float lo = (256.0f * c - 0.5f - kCellHalf) / kCellScale - kCellSlop;
+        const float hi = (256.0f * c + 255.5f - kCellHalf) / kCellScale + kCellSlop;
         float bnd = 3.0e38f;
-        unsigned below = 0;
+        float below = 0.0f;
         for (int k = 0; k < n_bnd; ++k) {
             const float b = cb.b[k];
-            if (b < lo) ++below;
+            if (b < lo) below += 1.0f;
             else if (b <= hi) bnd = b;
         }
-        lut[c] = make_float2(bnd, __uint_as_float(below));
+        lut[i] = make_float2(bnd, below);
     }
 }
 
 // x: the block's 32 input values (16-byte aligned).  w: packed codes (4 * BITS bytes, LSB-first), returns the
-// f32 scale (before the outlier sign).  cb: the outlier codebook of BITS bits.  lut: the 3-bit cell table in
-// shared memory (build_cell_table), or nullptr for the register bisection.  TABLE: the codebook is not the
+// f32 scale (before the outlier sign).  cb: the codebook.  lut: the caller's lane of the cell table in
+// shared memory (build_cell_table, + lane), or nullptr for the register bisection.  TABLE: the codebook is not the
 // 4-bit uniform grid even when BITS = 4 (codes of a narrower codebook stored at BITS width); needs lut.
+// Two values per instruction throughout (elements i and i + 16); the codes are whole f32 numbers that are packed by
+// multiply-adds (16 or 24 bits of them are exact) instead of a mask, a shift and an add each.
 template <typename T, int BITS, bool TABLE = false>
 __device__ __forceinline__ float pqo_quantize_block(const T* x, const Codebook& cb, float outer_centroid, uint32_t (&w)[4],
                                                     const float2* lut = nullptr) {
     const float inv_sqrt = 1.0f / sqrtf((float)kBlock);
     const float R = cb.c[(1 << BITS) - 1];
     const float inv_step = 15.0f / (2.0f * R);
-    float v[32];
-    load32<T>(x, v);
-    butterfly32_regs(v);
+    const float kMagic = 12582912.0f;          // 1.5 * 2^23
+    F2 p[16];
+    {
+        float v[32];
+        load32<T>(x, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) p[i] = f2(v[i], v[i + 16]);
+    }
+    butterfly32_pairs(p);
     float amax_w = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) amax_w = fmaxf(amax_w, fabsf(v[i]));
+    for (int i = 0; i < 16; ++i) {
+        const float2 t = halves(p[i]);
+        amax_w = fmaxf(amax_w, fmaxf(fabsf(t.x), fabsf(t.y)));
+    }
     const float amax = amax_w * inv_sqrt;          // rounding is monotone: equals max_i |W_i * inv_sqrt|
     const float raw = __fdiv_rn(amax, outer_centroid);
     const float scale = raw > kMinNorm ? raw : kMinNorm;
     const float r = __frcp_rn(scale);
-    w[0] = w[1] = w[2] = w[3] = 0u;
+    // (mag, mag) with the signs of elements i and i + 16
+    auto signed2 = [](F2 pp, F2 pn, F2 np, F2 nn, int i) {
+        return ((kSignMask >> i) & 1u) ? (((kSignMask >> (i + 16)) & 1u) ? nn : np) : (((kSignMask >> (i + 16)) & 1u) ? pn : pp);
+    };
+    F2 c[16];   // the codes
     if (BITS == 4 && !TABLE) {
         const float cpos = (inv_sqrt * r) * inv_step, cneg = -cpos;
-        const float kMagic = 12582912.0f;          // 1.5 * 2^23
-        bool near = false;
+        const F2 pp = f2(cpos, cpos), pn = f2(cpos, cneg), np = f2(cneg, cpos), nn = f2(cneg, cneg);
+        float far = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const float u = fmaf(v[i], ((kSignMask >> i) & 1u) ? cneg : cpos, 7.5f);
-            const float y = u + kMagic;
-            const float d = u - (y - kMagic);
-            near |= fabsf(d) > 0.49998f;
-            w[i >> 3] += (__float_as_uint(y) & 15u) << (4 * (i & 7));
+        for (int i = 0; i < 16; ++i) {
+            const F2 u = fma2(p[i], signed2(pp, pn, np, nn, i), f2(7.5f));
+            c[i] = add2(add2(u, f2(kMagic)), f2(-kMagic));
+            const float2 d = halves(sub2(u, c[i]));
+            far = fmaxf(far, fmaxf(fabsf(d.x), fabsf(d.y)));
         }
-        if (near) {   // rare: exact division and the f32 boundary table
-            w[0] = w[1] = w[2] = w[3] = 0u;
+        if (far > 0.49998f) {   // rare: exact division and the f32 boundary table
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const float rot = (v[i] * inv_sqrt) * (((kSignMask >> i) & 1u) ? -1.0f : 1.0f);
-                const float t = __fdiv_rn(rot, scale);
-                unsigned c = 0;
+            for (int i = 0; i < 16; ++i) {
+                const float2 v = halves(p[i]);
+                const float t0 = __fdiv_rn((v.x * inv_sqrt) * (((kSignMask >> i) & 1u) ? -1.0f : 1.0f), scale);
+                const float t1 = __fdiv_rn((v.y * inv_sqrt) * (((kSignMask >> (i + 16)) & 1u) ? -1.0f : 1.0f), scale);
+                float c0 = 0.0f, c1 = 0.0f;
 #pragma unroll
-                for (int k = 0; k < 15; ++k) c += (t > cb.b[k]) ? 1u : 0u;
-                w[i >> 3] += c << (4 * (i & 7));
+                for (int k = 0; k < 15; ++k) {
+                    c0 += (t0 > cb.b[k]) ? 1.0f : 0.0f;
+                    c1 += (t1 > cb.b[k]) ? 1.0f : 0.0f;
+                }
+                c[i] = f2(c0, c1);
             }
         }
     } else {
+        const F2 pp = f2(inv_sqrt, inv_sqrt), pn = f2(inv_sqrt, -inv_sqrt), np = f2(-inv_sqrt, inv_sqrt), nn = f2(-inv_sqrt, -inv_sqrt);
+        const F2 r2 = f2(r), ns2 = f2(-scale);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const float rot = v[i] * (((kSignMask >> i) & 1u) ? -inv_sqrt : inv_sqrt);
-            const float q = rot * r;
-            const float rem = fmaf(-q, scale, rot);
-            const float t = fmaf(rem, r, q);           // == rot / scale, correctly rounded
-            unsigned c;
+        for (int i = 0; i < 16; ++i) {
+            const F2 rot = mul2(p[i], signed2(pp, pn, np, nn, i));
+            const F2 q = mul2(rot, r2);
+            const F2 rem = fma2(q, ns2, rot);
+            const float2 t = halves(fma2(rem, r2, q));           // == rot / scale, correctly rounded
             if (lut != nullptr) {
-                const float y = fmaf(q, kCellScale, kCellHalf + 12582912.0f);   // round to nearest cell
-                const float2 e = lut[__float_as_uint(y) & 255u];
-                c = __float_as_uint(e.y) + (t > e.x ? 1u : 0u);
+                const float2 y = halves(fma2(q, f2(kCellScale), f2(kCellHalf + kMagic)));   // k in the low mantissa bits
+                // byte offset of [k >> 8][lane]: a cell row is 256 bytes
+                const unsigned char* l = reinterpret_cast<const unsigned char*>(lut);
+                const float2 e0 = *reinterpret_cast<const float2*>(l + (__float_as_uint(y.x) & ((kCells - 1) << 8)));
+                const float2 e1 = *reinterpret_cast<const float2*>(l + (__float_as_uint(y.y) & ((kCells - 1) << 8)));
+                c[i] = add2(f2(e0.y, e1.y), f2(t.x > e0.x ? 1.0f : 0.0f, t.y > e1.x ? 1.0f : 0.0f));
             } else {
                 // bisection over the 7 boundaries (constant bank operands)
-                const bool p1 = t > cb.b[3];
-                const bool p2 = t > (p1 ? cb.b[5] : cb.b[1]);
-                const float t3 = p1 ? (p2 ? cb.b[6] : cb.b[4]) : (p2 ? cb.b[2] : cb.b[0]);
-                const bool p3 = t > t3;
-                c = (p1 ? 4u : 0u) + (p2 ? 2u : 0u) + (p3 ? 1u : 0u);
+                float code[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float th = h == 0 ? t.x : t.y;
+                    const bool p1 = th > cb.b[3];
+                    const bool p2 = th > (p1 ? cb.b[5] : cb.b[1]);
+                    const float t3 = p1 ? (p2 ? cb.b[6] : cb.b[4]) : (p2 ? cb.b[2] : cb.b[0]);
+                    code[h] = (p1 ? 4.0f : 0.0f) + (p2 ? 2.0f : 0.0f) + (th > t3 ? 1.0f : 0.0f);
+                }
+                c[i] = f2(code[0], code[1]);
             }
-            const int bit = BITS * i;
-            w[bit >> 5] += c << (bit & 31);
-            if ((bit & 31) + BITS > 32) w[(bit >> 5) + 1] += c >> (32 - (bit & 31));
         }
+    }
+    if (BITS == 4) {
+        uint32_t h[2][4];   // [codes 0..15 | 16..31][four codes in the low 16 bits]
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            F2 a = fma2(c[4 * m + 3], f2(16.0f), c[4 * m + 2]);
+            a = fma2(a, f2(16.0f), c[4 * m + 1]);
+            a = add2(fma2(a, f2(16.0f), c[4 * m]), f2(8388608.0f));
+            const float2 t = halves(a);
+            h[0][m] = __float_as_uint(t.x);
+            h[1][m] = __float_as_uint(t.y);
+        }
+        w[0] = __byte_perm(h[0][0], h[0][1], 0x5410);
+        w[1] = __byte_perm(h[0][2], h[0][3], 0x5410);
+        w[2] = __byte_perm(h[1][0], h[1][1], 0x5410);
+        w[3] = __byte_perm(h[1][2], h[1][3], 0x5410);
+    } else {
+        F2 a = c[7], b = c[15];   // eight codes, 24 bits: below 2^24, exact
+#pragma unroll
+        for (int i = 6; i >= 0; --i) {
+            a = fma2(a, f2(8.0f), c[i]);
+            b = fma2(b, f2(8.0f), c[i + 8]);
+        }
+        const float2 ta = halves(a), tb = halves(b);
+        const uint32_t c0 = __float2uint_rz(ta.x), c1 = __float2uint_rz(tb.x), c2 = __float2uint_rz(ta.y), c3 = __float2uint_rz(tb.y);
+        w[0] = c0 | (c1 << 24);
+        w[1] = (c1 >> 8) | (c2 << 16);
+        w[2] = (c2 >> 16) | (c3 << 8);
+        w[3] = 0u;
     }
     return scale;
 }
