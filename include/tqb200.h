@@ -397,6 +397,12 @@ int tqb_pqo_cache_host_sync(tqb_pqo_cache *c);
 int tqb_pqo_cache_prefill_attend(tqb_pqo_cache *c, int32_t layer, const void *k, const void *v, const void *q,
                                  int32_t dtype, int32_t new_tokens, int32_t num_q_heads, float softmax_scale,
                                  void *out, tqb_stream_t stream);
+/* The same with q and out laid out [batch, num_q_heads, new_tokens, head_dim], as projections leave them: the kernel reads and
+ * writes them where they lie.  Shapes that tqb_chunk_attention would fold into decode launches return
+ * TQB_ERR_UNSUPPORTED with nothing stored. */
+int tqb_pqo_cache_prefill_attend_heads(tqb_pqo_cache *c, int32_t layer, const void *k, const void *v, const void *q,
+                                       int32_t dtype, int32_t new_tokens, int32_t num_q_heads, float softmax_scale,
+                                       void *out, tqb_stream_t stream);
 
 /* dequantize_full (pqo.rs:176-180): [batch, num_kv_heads, seq_len, head_dim] of `dtype`. */
 int tqb_pqo_cache_dequantize_full(tqb_pqo_cache *c, int32_t layer, void *k_out, void *v_out, int32_t dtype,

@@ -521,3 +521,37 @@ def test_pqo_cache_prefill_attend_two_chunks_then_decode(bits):
     q1 = (torch.randn((b, hq, 1, d), generator=g) / d ** 0.5).bfloat16().cuda()
     dec = cache.decode(0, k1, k1, q1, tq.AttendConfig(softmax_scale=scale, n_kv_groups=hq // hkv))
     assert dec.is_fused() and cache.seq_len(0) == 58 and torch.isfinite(dec.fused.float()).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("bits,batch,hq,hkv,tokens", [(4, 1, 8, 2, (1, 129, 40)), (3, 3, 4, 4, (33, 31)), (4, 2, 16, 2, (17, 200)), (4, 2, 6, 2, (30, 5))])
+def test_prefill_attend_reads_queries_where_they_lie(bits, batch, hq, hkv, tokens, dtype):
+    # [batch, heads, tokens, head_dim] in and out, chunk after chunk, against the folded path over the cache's own bytes
+    # (a group of 3 query heads takes the folded path inside the cache too)
+    g = torch.Generator(device="cuda").manual_seed(hq + batch)
+    cache = tq.PqoCache(tq.CacheConfig(bits=bits, head_dim=128, num_kv_heads=hkv, num_layers=1, batch=batch))
+    n = 0
+    for t in tokens:
+        k, v = (torch.randn((batch, hkv, t, 128), generator=g, device="cuda").to(dtype) for _ in range(2))
+        q = (torch.randn((batch, hq, t, 128), generator=g, device="cuda")).to(dtype)
+        out = cache.prefill_attend(0, k, v, q, tq.AttendConfig(0.09, hq // hkv))
+        n += t
+        assert out.shape == q.shape and out.is_contiguous() and cache.seq_len(0) == n
+        ki, ks, vi, vs = cache.export_layer(0, host=False)
+        rows = q.permute(2, 0, 1, 3).reshape(t, batch * hq, 128)
+        want = tq.chunk_attention(rows, ki, ks, vi, vs, n, bits, 0.09, fold=True, out_dtype=torch.float32).view(t, batch, hq, 128).permute(1, 2, 0, 3)
+        # f16 operands on the tensor cores (TOL), and the outputs' own rounding
+        assert ((out.float() - want).abs() <= TOL + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs()).all()
+
+
+def test_chunk_queries_off_a_16_byte_boundary():
+    g = torch.Generator(device="cuda").manual_seed(3)
+    hkv, hq, n, t = 2, 8, 300, 45
+    arrays = []
+    for _ in range(2):
+        i, s = tq.block_quantize(torch.randn((hkv * n, 128), generator=g, device="cuda"), 4)
+        arrays += [i.view(hkv, n, -1), s.view(hkv, n, -1)]
+    for dtype in (torch.float32, torch.float16):
+        hold = torch.randn(t * hq * 128 + 1, generator=g, device="cuda").to(dtype)
+        q = hold[1:].view(t, hq, 128)
+        assert torch.equal(tq.chunk_attention(q, *arrays, n, 4, 0.09), tq.chunk_attention(q.clone(), *arrays, n, 4, 0.09))

@@ -17,6 +17,7 @@ import torch
 from ._lib import TqbCacheConfig, TqbConfig, TqbDecodeParams, lib
 
 TQB_F32, TQB_F16, TQB_BF16 = 0, 1, 2
+TQB_ERR_UNSUPPORTED = 9
 ALL_BLOCKS = -1  # usize::MAX in src/cache/config.rs:49-50
 DEFAULT_ROTATION_SEED = 42   # src/cache/config.rs:15
 DEFAULT_QJL_SEED = 12345     # src/cache/config.rs:18
@@ -683,6 +684,14 @@ class PqoCache:
         k, v [batch, Hkv, T, D]; q [batch, Hq, T, D] (device tensors); returns [batch, Hq, T, D]."""
         k, v = k.contiguous(), v.contiguous()
         b, hq, t, d = q.shape
+        q = q.contiguous()
+        out = torch.empty_like(q)
+        st = lib.tqb_pqo_cache_prefill_attend_heads(self._h, layer, _ptr(k), _ptr(v), _ptr(q), _dtype_code(k.dtype), t, hq,
+                                                    config.softmax_scale, _ptr(out), _stream())
+        if st != TQB_ERR_UNSUPPORTED:
+            check(st)
+            return out
+        # the folded path takes its queries token by token
         qt = q.permute(2, 0, 1, 3).contiguous()            # [T, batch * Hq, D]
         out = torch.empty_like(qt)
         check(lib.tqb_pqo_cache_prefill_attend(self._h, layer, _ptr(k), _ptr(v), _ptr(qt), _dtype_code(k.dtype), t, hq,

@@ -28,7 +28,7 @@ int launch_decode_mma(const tqb_decode_params* p, int num_partitions, float* par
                       const int* gate = nullptr, int gate_want = 0, const float* dev_signs = nullptr, int alias_heads = 0,
                       const PeerPush* peer = nullptr, float* group_area = nullptr);
 
-int launch_chunk_umma(const tqb_decode_params* p, int q_len, cudaStream_t s);
+int launch_chunk_umma(const tqb_decode_params* p, int q_len, cudaStream_t s, size_t q_tok, size_t q_head);
 
 namespace {
 
@@ -560,7 +560,7 @@ int tqb_chunk_attention(const tqb_decode_params* p, int32_t q_len, tqb_stream_t 
         if (p->num_q_heads % p->num_kv_heads != 0) return TQB_ERR_INVALID_ARGUMENT;
         if (p->kv_len > p->kv_stride) return TQB_ERR_RANGE_OUT_OF_BOUNDS;
         if (!p->k_indices || !p->k_scales || !p->v_indices || !p->v_scales) return TQB_ERR_NULL_POINTER;
-        const int st = launch_chunk_umma(p, q_len, as_stream(stream));
+        const int st = launch_chunk_umma(p, q_len, as_stream(stream), 0, 0);
         if (st != TQB_ERR_UNSUPPORTED) return st;
     }
     tqb_decode_params f = *p;

@@ -19,6 +19,10 @@
 // the even and the odd tiles, merged once at the end like two split-K partitions.  Thread r of a group owns query
 // row r = tensor-memory lane r, so the online softmax needs no shuffles; the output is rotated back in registers
 // (one 32-point butterfly per block) at the end.
+// Measured (B200, 32 q / 8 KV heads, 4-bit, bf16): 512 queries on 7,680 tokens 98 us = 670 TFLOP/s of causal attention math.
+// It took 134 us with the queries rotated a warp per block (34 dependent loads before the first tile), one f32
+// operation an instruction in the softmax, and the CTAs started in ascending order of their work; a 1,999-token prompt's
+// call (store + attend) went from 120 - 150 to 67 us, of which two transposing passes over q and out were 23.
 // The f16 roundings of Q~, K~, P and V are this kernel's error budget (a few 1e-4 of the value range on the outputs;
 // the decode kernels, which keep the query in f32 or as 20-bit integers, stay below 1e-5).
 //
@@ -31,6 +35,8 @@
 #include <atomic>
 
 #include "tqb_common.cuh"
+#include "tqb_f32x2.cuh"
+#include "tqb_pqo_quant.cuh"
 
 namespace tqb {
 namespace {
@@ -39,26 +45,23 @@ constexpr int kRows = 128;          // query rows per CTA
 constexpr int kTile = 64;           // cache tokens per step
 constexpr int kD = 128;
 constexpr int kThreads = 15 * 32;
-// P = exp2(s - m) goes to the tensor cores through tensor memory: a softmax thread overwrites the first 32 columns of
-// the 64 score columns it has just read with its row of P (two f16 per column), and the P V product takes its A operand
-// from there.  (false: through shared memory, as a K-major swizzled tile.)
-constexpr bool kPTmem = true;
 constexpr float kNegBig = -1.0e30f;
 
 // shared-memory map (bytes from a 1024-aligned base)
 constexpr int kOffQ = 0;                         // [2 atoms][128 rows][128 B]
 constexpr int kOffK = 32768;                     // [2 stages][2 atoms][128 tokens = two tiles][128 B]
 constexpr int kOffV = kOffK + 2 * 32768;         // [2 stages][2 dim halves][8 token groups][8 tokens][128 B]
-constexpr int kOffP = kOffV + 2 * 16384;         // [2 buffers][128 rows][128 B]
-constexpr int kOffLut = kOffP + 2 * 16384;       // 3-bit: 64 half2
+constexpr int kOffLut = kOffV + 2 * 16384;       // 3-bit: 64 half2
 constexpr int kOffBar = kOffLut + 256;           // mbarriers
 constexpr int kOffMl = kOffBar + 128;            // (max, sum) of every row of both softmax groups, for the final merge
 constexpr int kSmemBytes = kOffMl + 2048 + 1024; // + alignment slack
 constexpr uint32_t kTmemCols = 512;              // S buffers (128 columns: two tiles) at 0 and 128; O of group 0 at 256, of group 1 at 384
 
 struct ChunkArgs {
-    const void* q;        // [q_len, hq, 128]
-    void* out;            // [q_len, hq, 128]
+    const void* q;        // [q_len, hq, 128]: element strides q_tok and q_head
+    void* out;            // same strides
+    size_t q_tok, q_head;
+    bool q_wide, out_wide;   // 16-byte aligned: vector accesses
     float* lse_out;       // nullptr or [q_len, hq, 2]
     const uint8_t* kb;
     const uint16_t* ks;
@@ -201,14 +204,6 @@ __device__ __forceinline__ void nibbles_to_half2(uint32_t w, uint32_t (&x)[4]) {
 // Position p (0..7) inside a group of eight unpacked 4-bit codes holds code kPerm4[p] of the word.
 __device__ __forceinline__ int perm4(int p) { return (p >> 1) + 4 * (p & 1); }
 
-__device__ __forceinline__ float wht32_lane(float v, int lane) {
-#pragma unroll
-    for (int h = 1; h < 32; h <<= 1) {
-        float other = __shfl_xor_sync(0xffffffffu, v, h);
-        v = (lane & h) ? (other - v) : (v + other);
-    }
-    return v;
-}
 
 // 16 consecutive bytes of a swizzled 128-byte row: chunk c of row `row` of a tile whose rows are 128 bytes apart
 __device__ __forceinline__ uint32_t sw128(int row, int chunk) { return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4)); }
@@ -301,7 +296,8 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
     __shared__ int s_fail;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = a.g, TQ = kRows / g;
-    const int mt = blockIdx.x, kvh = blockIdx.y;
+    // the query tiles that see most of the cache first, over all heads: what is left for the last CTAs is short
+    const int kvh = blockIdx.x % a.hkv, mt = (gridDim.x - 1 - blockIdx.x) / a.hkv;
     const int tok0 = mt * TQ;                                   // first query token of the tile
     const int ntok = min(TQ, a.q_len - tok0);                   // valid query tokens in the tile
     const int past = a.kv_len - a.q_len;                        // tokens before the chunk
@@ -337,27 +333,46 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
             reinterpret_cast<__half2*>(sm + kOffLut)[e] = __floats2half2_rn(a.lut[e & 7], a.lut[e >> 3]);
     }
     // ---- rotated queries -> Q tile (K-major, 128-byte swizzle, two atoms of 64 dims), rounded to f16 ----
-    {
-        const uint32_t neg = 0xB1A6D4B2u;   // src/cache/precomputed/rotation.rs:16-20
-        const float sign = ((neg >> lane) & 1u) ? -a.sign_mag : a.sign_mag;
-        const float inv_sqrt = 1.0f / sqrtf(32.0f);
-        for (int u = warp; u < kRows * 4; u += kThreads / 32) {
-            const int r = u >> 2, b = u & 3;
-            const int tq = r / g, hh = r - tq * g;
-            float v = 0.0f;
-            if (tq < ntok)
-                v = to_f32<QT>(reinterpret_cast<const QT*>(a.q)[((size_t)(tok0 + tq) * a.hq + kvh * g + hh) * kD + b * 32 + lane]);
-            v = wht32_lane(v, lane);
-            v = ((v * inv_sqrt) * sign) * a.qk_const;
-            // position of dim (b, lane) inside the K tile's element order
-            int pos = lane;
-            if (BITS == 4) {   // word j = lane / 8 holds codes in the order c0, c4, c1, c5, ...: code k sits at position
-                const int k = lane & 7;
-                pos = (lane & ~7) | ((k & 3) * 2 + (k >> 2));
+    // One thread takes a 32-block of a row: its loads are in flight together and the butterfly stays in registers.  (A warp per
+    // block, one element a lane, waited for 34 loads one after the other before the first tile was touched.)
+    for (int u = tid; u < kRows * 4; u += kThreads) {
+        const int r = u >> 2, b = u & 3;
+        const int tq = r / g, hh = r - tq * g;
+        F2 p[16];
+        if (tq < ntok) {
+            float v[32];
+            const QT* src = reinterpret_cast<const QT*>(a.q) + ((size_t)(tok0 + tq) * a.q_tok + (size_t)(kvh * g + hh) * a.q_head) + b * 32;
+            if (a.q_wide) {
+                load32<QT>(src, v);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] = to_f32<QT>(src[i]);
             }
-            const int d = b * 32 + pos;
-            const uint32_t off = (uint32_t)(d >> 6) * 16384u + sw128(r, (d & 63) >> 3) + (uint32_t)(d & 7) * 2u;
-            *reinterpret_cast<__half*>(sm + kOffQ + off) = __float2half_rn(v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) p[i] = f2(v[i], v[i + 16]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) p[i] = f2(0.0f);
+        }
+        butterfly32_pairs(p);
+        const float inv_sqrt = 1.0f / sqrtf(32.0f);
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float s0 = ((kSignMask >> i) & 1u) ? -a.sign_mag : a.sign_mag, s1 = ((kSignMask >> (i + 16)) & 1u) ? -a.sign_mag : a.sign_mag;
+            const float2 t = halves(mul2(mul2(mul2(p[i], f2(inv_sqrt)), f2(s0, s1)), f2(a.qk_const)));
+            v[i] = t.x;
+            v[i + 16] = t.y;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            // position e of a group of eight holds, like the K tile, dim perm4(e) (4-bit) or e
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                w[e] = h2_as_u32(BITS == 4 ? __floats2half2_rn(v[8 * j + perm4(2 * e)], v[8 * j + perm4(2 * e + 1)])
+                                           : __floats2half2_rn(v[8 * j + 2 * e], v[8 * j + 2 * e + 1]));
+            *reinterpret_cast<uint4*>(sm + kOffQ + (b >> 1) * 16384 + sw128(r, 4 * (b & 1) + j)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     }
     fence_async_smem();
@@ -379,7 +394,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
             // Descriptors are built once: inside the loops a descriptor is its base plus a compile-time offset in the
             // address field (bytes >> 4), so that the one issuing thread spends a handful of instructions per MMA.
             const uint64_t dQ = umma_desc(base + kOffQ, 16, 1024), dK = umma_desc(base + kOffK, 16, 1024);
-            const uint64_t dP = umma_desc(base + kOffP, 16, 1024), dV = umma_desc(base + kOffV, 8192, 1024);
+            const uint64_t dV = umma_desc(base + kOffV, 8192, 1024);
             // S(j) = Q~ K~^T for the 128 tokens of step j: 8 k-steps of 16 dims (atom = 64 dims = 16 KB, 32 bytes per
             // k-step), N = 128
             auto score = [&](int j) -> bool {
@@ -408,14 +423,11 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
                     if (!mbar_wait(bar + kVFull + 8 * G, j & 1, (2u << 24) | (1u << 16) | (unsigned)j)) { ok = false; break; }
                     tc_fence_after();
                     // O_G += P V : four k-steps of 16 tokens
-                    const uint64_t pv = dP + (uint64_t)(G * (16384 >> 4)), vv = dV + (uint64_t)(G * (16384 >> 4));
+                    const uint64_t vv = dV + (uint64_t)(G * (16384 >> 4));
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk) {
-                        if (kPTmem)
-                            umma_f16_ts(tmemO + G * kD, tmemS + (j & 1) * 2 * kTile + G * kTile + kk * 8, vv + (uint64_t)((kk * 2048) >> 4),
-                                        idescO, (j | kk) ? 1u : 0u);
-                        else
-                            umma_f16(tmemO + G * kD, pv + (uint64_t)((kk * 32) >> 4), vv + (uint64_t)((kk * 2048) >> 4), idescO, (j | kk) ? 1u : 0u);
+                        umma_f16_ts(tmemO + G * kD, tmemS + (j & 1) * 2 * kTile + G * kTile + kk * 8, vv + (uint64_t)((kk * 2048) >> 4),
+                                    idescO, (j | kk) ? 1u : 0u);
                     }
                     umma_commit(bar + kVEmpty + 8 * G);      // frees this V stage and P buffer when the MMAs issued so far are done
                 }
@@ -450,40 +462,41 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
                 tmem_ld32(tmemS + lane_base + sb * 2 * kTile + G * kTile, v0);
                 tmem_ld32(tmemS + lane_base + sb * 2 * kTile + G * kTile + 32, v1);
                 tmem_wait_ld();
-                if ((i + 1) * kTile <= limit_min) {
-                    // every token of the tile is visible to every row (all tiles but the last few)
 #pragma unroll
-                    for (int t = 0; t < 32; ++t) {
-                        p[t] = __uint_as_float(v0[t]);
-                        p[32 + t] = __uint_as_float(v1[t]);
-                    }
-                } else {
+                for (int t = 0; t < 32; ++t) {
+                    p[t] = __uint_as_float(v0[t]);
+                    p[32 + t] = __uint_as_float(v1[t]);
+                }
+                if ((i + 1) * kTile > limit_min) {   // the last few tiles: tokens that a row does not see yet
+                    const int seen = row_valid ? limit - i * kTile : 0;
 #pragma unroll
-                    for (int t = 0; t < 32; ++t) {
-                        const int tok = i * kTile + t;
-                        p[t] = (row_valid && tok < limit) ? __uint_as_float(v0[t]) : kNegBig;
-                        p[32 + t] = (row_valid && tok + 32 < limit) ? __uint_as_float(v1[t]) : kNegBig;
-                    }
+                    for (int t = 0; t < kTile; ++t) p[t] = t < seen ? p[t] : kNegBig;
                 }
             }
             // four interleaved partial maxima / sums keep the dependency chains short
             float mx4[4] = {kNegBig, kNegBig, kNegBig, kNegBig};
 #pragma unroll
-            for (int t = 0; t < kTile; ++t) mx4[t & 3] = fmaxf(mx4[t & 3], p[t]);
+            for (int t = 0; t < kTile; t += 8)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(fmaxf(mx4[e], p[t + 2 * e]), p[t + 2 * e + 1]);
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
             // lazy maximum: raise the reference only when this tile exceeds it by more than 2^6.  A row that has seen no
             // visible token yet keeps the sentinel; the floor below then turns its masked scores into exp2(-huge) = 0.
             const float m_new = (mx - m_run > 6.0f) ? mx : m_run;
             const float resc = ex2(m_run - m_new);
-            const float m_use = fmaxf(m_new, -1.0e29f);
+            const F2 m_use = f2(-fmaxf(m_new, -1.0e29f));
             m_run = m_new;
-            float ls4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            F2 ls[4] = {f2(0.0f), f2(0.0f), f2(0.0f), f2(0.0f)};
+            uint32_t w[kTile / 2];   // P: tokens 2c (low half) and 2c + 1
 #pragma unroll
-            for (int t = 0; t < kTile; ++t) {
-                p[t] = ex2(p[t] - m_use);
-                ls4[t & 3] += p[t];
+            for (int c = 0; c < kTile / 2; ++c) {
+                const float2 d = halves(add2(f2(p[2 * c], p[2 * c + 1]), m_use));
+                const float e0 = ex2(d.x), e1 = ex2(d.y);
+                ls[c & 3] = add2(ls[c & 3], f2(e0, e1));
+                w[c] = h2_as_u32(__floats2half2_rn(e0, e1));
             }
-            l_run = l_run * resc + ((ls4[0] + ls4[1]) + (ls4[2] + ls4[3]));
+            const float2 lt = halves(add2(add2(ls[0], ls[1]), add2(ls[2], ls[3])));
+            l_run = l_run * resc + (lt.x + lt.y);
             // The group's P V product of the previous step must be done: it wrote the O accumulator rescaled here (and,
             // with P in shared memory, read the P buffer written below).  The wait is also the flow control of the
             // p_full barrier: without it a group could arrive for steps j and j + 1 before the issuing thread has looked
@@ -505,25 +518,9 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
                 }
                 tmem_wait_st();
             }
-            if (kPTmem) {
-                // P -> tensor memory: column c of the row holds tokens 2c (low half) and 2c + 1
-                uint32_t w[32];
-#pragma unroll
-                for (int c = 0; c < 32; ++c) w[c] = h2_as_u32(__floats2half2_rn(p[2 * c], p[2 * c + 1]));
-                tmem_st32(tmemS + lane_base + sb * 2 * kTile + G * kTile, w);
-                tmem_wait_st();
-            } else {
-                // P -> shared memory (K-major A operand: row r, 64 tokens = 128 bytes, swizzled 16-byte chunks)
-                unsigned char* pt = sm + kOffP + G * 16384;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) w[e] = h2_as_u32(__floats2half2_rn(p[8 * c + 2 * e], p[8 * c + 2 * e + 1]));
-                    *reinterpret_cast<uint4*>(pt + sw128(r, c)) = make_uint4(w[0], w[1], w[2], w[3]);
-                }
-                fence_async_smem();
-            }
+            // P -> tensor memory: column c of the row holds tokens 2c and 2c + 1
+            tmem_st32(tmemS + lane_base + sb * 2 * kTile + G * kTile, w);
+            tmem_wait_st();
             tc_fence_before();
             mbar_arrive(bar + kPFull + 8 * G);
         }
@@ -546,7 +543,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
             const float inv_l = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
             const float inv_sqrt = 1.0f / sqrtf(32.0f);
             const uint32_t neg = 0xB1A6D4B2u;
-            const size_t orow = ((size_t)(tok0 + tq) * a.hq + kvh * g + hh) * kD;
+            const size_t orow = (size_t)(tok0 + tq) * a.q_tok + (size_t)(kvh * g + hh) * a.q_head;
 #pragma unroll 1
             for (int b = 2 * G; b < 2 * G + 2; ++b) {
                 uint32_t va[32], vb[32];
@@ -571,15 +568,38 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
                             x[jx] = xa + xb;
                             x[jx + h] = xa - xb;
                         }
+                const float fin = a.lse_out == nullptr ? inv_l : 1.0f;
 #pragma unroll
-                for (int d = 0; d < 32; ++d) {
-                    float o = x[d] * inv_sqrt;
-                    if (a.lse_out == nullptr) o *= inv_l;
-                    const size_t idx = orow + b * 32 + d;
-                    if (!row_valid) continue;
-                    if (a.out_dtype == TQB_F32) reinterpret_cast<float*>(a.out)[idx] = o;
-                    else if (a.out_dtype == TQB_F16) reinterpret_cast<__half*>(a.out)[idx] = __float2half_rn(o);
-                    else reinterpret_cast<__nv_bfloat16*>(a.out)[idx] = __float2bfloat16_rn(o);
+                for (int d = 0; d < 32; ++d) x[d] = (x[d] * inv_sqrt) * fin;
+                if (!row_valid) continue;
+                const size_t idx = orow + b * 32;
+                if (!a.out_wide) {
+#pragma unroll
+                    for (int d = 0; d < 32; ++d) {
+                        if (a.out_dtype == TQB_F32) reinterpret_cast<float*>(a.out)[idx + d] = x[d];
+                        else if (a.out_dtype == TQB_F16) reinterpret_cast<__half*>(a.out)[idx + d] = __float2half_rn(x[d]);
+                        else reinterpret_cast<__nv_bfloat16*>(a.out)[idx + d] = __float2bfloat16_rn(x[d]);
+                    }
+                } else if (a.out_dtype == TQB_F32) {
+                    float4* o4 = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + idx);
+#pragma unroll
+                    for (int d = 0; d < 8; ++d) o4[d] = make_float4(x[4 * d], x[4 * d + 1], x[4 * d + 2], x[4 * d + 3]);
+                } else {
+                    uint4* o4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.out) + idx);
+#pragma unroll
+                    for (int d = 0; d < 4; ++d) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float lo = x[8 * d + 2 * e], hi = x[8 * d + 2 * e + 1];
+                            if (a.out_dtype == TQB_F16) w[e] = h2_as_u32(__floats2half2_rn(lo, hi));
+                            else {
+                                __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+                                w[e] = *reinterpret_cast<uint32_t*>(&h);
+                            }
+                        }
+                        o4[d] = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
                 }
             }
             if (a.lse_out != nullptr && row_valid && G == 0) {
@@ -632,22 +652,29 @@ int launch_chunk(const ChunkArgs& a, dim3 grid, cudaStream_t s) {
 
 }  // namespace
 
-// TQB_ERR_UNSUPPORTED when the shape is outside what this kernel covers (the caller then folds the chunk into decode launches).
-int launch_chunk_umma(const tqb_decode_params* p, int q_len, cudaStream_t s) {
+// The shapes that the kernel covers (others: the caller folds the chunk into decode launches).
+bool chunk_umma_covers(const tqb_decode_params* p, int q_len) {
     const int nblk = p->head_dim / kBlock;
     const int g = p->num_kv_heads > 0 ? p->num_q_heads / p->num_kv_heads : 0;
     const bool all_outlier = p->outlier_blocks < 0 || p->outlier_blocks >= nblk;
-    const bool all_normal = p->outlier_blocks == 0;
-    if (p->head_dim != kD || p->qjl_enabled || p->kv_len <= 0 || q_len <= 0) return TQB_ERR_UNSUPPORTED;
-    if (g != 1 && g != 2 && g != 4 && g != 8) return TQB_ERR_UNSUPPORTED;
-    const bool pqo4 = p->bits == 4 && p->norm_mode == TQB_MAXNORM && all_outlier;
-    const bool lut3 = p->bits == 3 && (all_outlier || all_normal);
-    if (!pqo4 && !lut3) return TQB_ERR_UNSUPPORTED;
-    if (((uintptr_t)p->k_indices % 16) || ((uintptr_t)p->v_indices % 16) || ((uintptr_t)p->k_scales % 8) || ((uintptr_t)p->v_scales % 8))
-        return TQB_ERR_UNSUPPORTED;
+    if (p->head_dim != kD || p->qjl_enabled || p->kv_len <= 0 || q_len <= 0) return false;
+    if (g != 1 && g != 2 && g != 4 && g != 8) return false;
+    if (!(p->bits == 4 && p->norm_mode == TQB_MAXNORM && all_outlier) && !(p->bits == 3 && (all_outlier || p->outlier_blocks == 0))) return false;
+    return !(((uintptr_t)p->k_indices % 16) || ((uintptr_t)p->v_indices % 16) || ((uintptr_t)p->k_scales % 8) || ((uintptr_t)p->v_scales % 8));
+}
+
+// q and out: element (token i, head h, d) at i * q_tok + h * q_head + d (q_tok = 0: [q_len, hq, 128]).
+int launch_chunk_umma(const tqb_decode_params* p, int q_len, cudaStream_t s, size_t q_tok, size_t q_head) {
+    if (!chunk_umma_covers(p, q_len)) return TQB_ERR_UNSUPPORTED;
+    const int g = p->num_q_heads / p->num_kv_heads;
+    const bool all_outlier = p->outlier_blocks < 0 || p->outlier_blocks >= p->head_dim / kBlock;
     if (p->lse_out && p->out_dtype != TQB_F32) return TQB_ERR_INVALID_ARGUMENT;
     ChunkArgs a{};
     a.q = p->q; a.out = p->out; a.lse_out = p->lse_out;
+    a.q_tok = q_tok ? q_tok : (size_t)p->num_q_heads * kD;
+    a.q_head = q_tok ? q_head : kD;
+    a.q_wide = ((uintptr_t)p->q % 16) == 0;
+    a.out_wide = ((uintptr_t)p->out % 16) == 0;
     a.kb = p->k_indices; a.ks = p->k_scales; a.vb = p->v_indices; a.vs = p->v_scales;
     a.hq = p->num_q_heads; a.hkv = p->num_kv_heads; a.g = g; a.q_len = q_len; a.kv_len = p->kv_len; a.kv_stride = p->kv_stride;
     a.out_dtype = p->out_dtype;
@@ -655,7 +682,7 @@ int launch_chunk_umma(const tqb_decode_params* p, int q_len, cudaStream_t s) {
     volatile float sq = sqrtf(32.0f);
     a.sign_mag = inv * sq;   // the reference's sign pattern: (1 / sqrt(32)) * sqrt(32) in f32
     const float log2e = 1.4426950408889634f;
-    if (pqo4) {
+    if (p->bits == 4) {
         const float step = (2.0f * 2.1573f) / 15.0f;   // src/cache/precomputed/codebooks.rs:64-67
         a.qk_const = p->softmax_scale * log2e * step;
         a.v_const = step;
@@ -687,7 +714,7 @@ int launch_chunk_umma(const tqb_decode_params* p, int q_len, cudaStream_t s) {
     if (cudaGetSymbolAddress(&tptr, g_chunk_timeouts) != cudaSuccess) return TQB_ERR_CUDA;
     a.timeouts = static_cast<unsigned*>(tptr);
     const int TQ = kRows / g;
-    dim3 grid((q_len + TQ - 1) / TQ, p->num_kv_heads);
+    dim3 grid((unsigned)((q_len + TQ - 1) / TQ) * (unsigned)p->num_kv_heads);
 #define TQB_LAUNCH_CHUNK(QT) (p->bits == 4 ? launch_chunk<QT, 4>(a, grid, s) : launch_chunk<QT, 3>(a, grid, s))
     if (p->q_dtype == TQB_F32) return TQB_LAUNCH_CHUNK(float);
     if (p->q_dtype == TQB_F16) return TQB_LAUNCH_CHUNK(__half);

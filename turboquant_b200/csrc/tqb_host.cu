@@ -336,10 +336,8 @@ struct tqb_pqo_cache {
         p.append_v = append_v;
         return tqb_decode_attention(&p, s);
     }
-    // Causal attention of the last q_len stored tokens' queries over the layer (q, out: [q_len, batch * Hq, D]).
-    int attend_chunk(int layer, const void* q_dev, int dtype, int num_q_heads, int q_len, float softmax_scale, void* out_dev,
-                     cudaStream_t s) {
-        Layer& l = layers[layer];
+    tqb_decode_params chunk_params(int layer, const void* q_dev, int dtype, int num_q_heads, float softmax_scale, void* out_dev) const {
+        const Layer& l = layers[layer];
         tqb_decode_params p{};
         p.q = q_dev;
         p.k_indices = l.ki; p.k_scales = l.ks; p.v_indices = l.vi; p.v_scales = l.vs;
@@ -351,8 +349,14 @@ struct tqb_pqo_cache {
         p.num_kv_heads = heads;
         p.kv_len = (int32_t)l.len;
         p.kv_stride = (int32_t)l.cap;
-        p.num_partitions = tqb_decode_num_partitions(heads * q_len, (int32_t)l.len);
         p.softmax_scale = softmax_scale;
+        return p;
+    }
+    // Causal attention of the last q_len stored tokens' queries over the layer (q, out: [q_len, batch * Hq, D]).
+    int attend_chunk(int layer, const void* q_dev, int dtype, int num_q_heads, int q_len, float softmax_scale, void* out_dev,
+                     cudaStream_t s) {
+        tqb_decode_params p = chunk_params(layer, q_dev, dtype, num_q_heads, softmax_scale, out_dev);
+        p.num_partitions = tqb_decode_num_partitions(heads * q_len, p.kv_len);
         const int folded = p.num_q_heads * q_len;
         const size_t need = tqb_decode_scratch_bytes(folded, cfg.head_dim, p.num_partitions);
         TQB_TRY(prepare_scratch(scratch, ticket_heads, need, folded, cfg.head_dim, p.num_partitions, s));
@@ -390,6 +394,8 @@ struct tqb_pqo_cache {
 };
 
 namespace tqb {
+bool chunk_umma_covers(const tqb_decode_params* p, int q_len);
+int launch_chunk_umma(const tqb_decode_params* p, int q_len, cudaStream_t s, size_t q_tok, size_t q_head);
 int peer_exchange_begin_step(tqb_peer_exchange* x, int num_q_heads, PeerPush& push, float** local_rec);
 }
 
@@ -469,6 +475,25 @@ int tqb_pqo_cache_prefill_attend(tqb_pqo_cache* c, int32_t layer, const void* k,
     cudaStream_t s = as_stream(stream);
     TQB_TRY(c->quantize_and_store(layer, k, v, dtype, new_tokens, s));
     return c->attend_chunk(layer, q, dtype, num_q_heads, new_tokens, softmax_scale, out, s);
+}
+
+int tqb_pqo_cache_prefill_attend_heads(tqb_pqo_cache* c, int32_t layer, const void* k, const void* v, const void* q, int32_t dtype,
+                                       int32_t new_tokens, int32_t num_q_heads, float softmax_scale, void* out,
+                                       tqb_stream_t stream) {
+    TQB_NVTX_RANGE();
+    TQB_TRY(check_layer(c, layer));
+    if (new_tokens <= 0) return TQB_ERR_INVALID_ARGUMENT;
+    if (dtype != TQB_F32 && dtype != TQB_F16 && dtype != TQB_BF16) return TQB_ERR_INVALID_ARGUMENT;
+    if (num_q_heads <= 0 || num_q_heads % c->cfg.num_kv_heads != 0) return TQB_ERR_INVALID_ARGUMENT;
+    if (!k || !v || !q || !out) return TQB_ERR_NULL_POINTER;
+    cudaStream_t s = as_stream(stream);
+    tqb_decode_params p = c->chunk_params(layer, q, dtype, num_q_heads, softmax_scale, out);
+    p.kv_len += new_tokens;
+    if (!chunk_umma_covers(&p, new_tokens)) return TQB_ERR_UNSUPPORTED;   // before anything is stored
+    if ((long long)p.num_q_heads * new_tokens > (1 << 24)) return TQB_ERR_TOO_LARGE;
+    TQB_TRY(c->quantize_and_store(layer, k, v, dtype, new_tokens, s));
+    p = c->chunk_params(layer, q, dtype, num_q_heads, softmax_scale, out);
+    return launch_chunk_umma(&p, new_tokens, s, (size_t)c->cfg.head_dim, (size_t)new_tokens * c->cfg.head_dim);
 }
 
 int tqb_pqo_cache_decode(tqb_pqo_cache* c, int32_t layer, const void* k, const void* v, const void* q, int32_t dtype,
