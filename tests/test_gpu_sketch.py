@@ -92,3 +92,29 @@ def test_projections_of_many_queries_equal_single_ones(dim):
     many = tq.query_projections(q, dim, 21)
     few = torch.cat([tq.query_projections(q[a:a + 100], dim, 21) for a in range(0, len(q), 100)])
     assert torch.equal(many.nan_to_num(7.0, 8.0, -8.0), few.nan_to_num(7.0, 8.0, -8.0))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("bits,dim,batch,group", [(3, 128, 1, 1), (3, 128, 5, 4), (4, 128, 3, 8), (3, 64, 2, 2), (4, 32, 1, 3), (3, 256, 2, 4)])
+def test_decode_input_in_one_launch_equals_separate_kernels(bits, dim, batch, group, dtype):
+    # a query that starts off a 16-byte boundary takes the separate kernels
+    hkv, steps = 2, 3
+    cfg = tq.CacheConfig(bits=bits, head_dim=dim, num_kv_heads=hkv, num_layers=1, batch=batch, outlier_blocks=0)
+    att, outs = tq.AttendConfig(dim ** -0.5, group), []
+    for shift in (0, 1):
+        g = torch.Generator(device="cuda").manual_seed(dim + batch)
+        cache = tq.TqCache(cfg)
+        got = []
+        for step in range(steps):
+            k, v = (torch.randn((batch, hkv, 1, dim), generator=g, device="cuda").to(dtype) for _ in range(2))
+            q = torch.randn((batch, hkv * group, 1, dim), generator=g, device="cuda").to(dtype)
+            if step == 1:
+                k[0, 0] = 0
+                k[-1, -1, 0, 3] = 1e4
+            hold = torch.zeros(q.numel() + shift, dtype=dtype, device="cuda")
+            hold[shift:] = q.reshape(-1)
+            got.append(cache.decode_fused(0, k, v, hold[shift:].view(q.shape), att).fused)
+        r = cache.decode(0, k, v, q).dequantized
+        outs.append(got + [r.k, r.v, r.logit_bias])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "tqb_common.cuh"
+#include "tqb_sketch.cuh"
 
 namespace {
 
@@ -1043,12 +1044,32 @@ struct tqb_tq_cache {
         return st;
     }
 
+    // One token per sequence, stored and its queries projected in one launch; TQB_ERR_UNSUPPORTED: nothing was done.
+    int store_one_and_project(int layer, const void* k, const void* v, const void* q, int dtype, int num_q_heads, cudaStream_t s) {
+        const auto& cfg = base->cfg;
+        if (cfg.norm_mode != TQB_MAXNORM || cfg.outlier_blocks != 0) return TQB_ERR_UNSUPPORTED;
+        const int64_t old_len = base->layers[layer].len;
+        const long long nq = (long long)cfg.batch * num_q_heads;
+        TQB_TRY(ensure_qjl_capacity(layer, old_len + 1, old_len, s));
+        TQB_TRY(rq.reserve((size_t)nq * cfg.head_dim * sizeof(float)));
+        TQB_TRY(base->ensure_capacity(layer, old_len + 1, s));
+        auto& L = base->layers[layer];
+        const TqAppend a{k, v, q, dtype, cfg.bits, cfg.head_dim, base->heads, nq, rbits, L.ki, L.vi, qjl[layer].signs,
+                         L.ks, L.vs, qjl[layer].norms, (long long)L.cap, (long long)qjl[layer].cap, (long long)old_len, (float*)rq.p};
+        TQB_TRY(launch_tq_append(a, s));
+        L.len = old_len + 1;
+        L.active = true;
+        return TQB_OK;
+    }
+
     // compute_logit_bias (src/cache/tq.rs:185-253)
     int project(const void* q, int dtype, int num_q_heads, int q_len, cudaStream_t s) {
         const long long nq = (long long)base->cfg.batch * num_q_heads * q_len;
         const size_t bytes = (size_t)nq * base->cfg.head_dim * sizeof(float);
-        TQB_TRY(qf32.reserve(bytes));
         TQB_TRY(rq.reserve(bytes));
+        if (nq >= kProjTileMin)
+            return launch_projections_tile(base->cfg.head_dim, q, dtype, nq, rbits, (float*)rq.p, 1.0f / sqrtf((float)base->cfg.head_dim), s);
+        TQB_TRY(qf32.reserve(bytes));
         TQB_TRY(convert_to_f32(q, dtype, (float*)qf32.p, nq * base->cfg.head_dim, s));
         return tqb_qjl_query_projections(base->cfg.head_dim, rbits, (const float*)qf32.p, nq, (float*)rq.p, s);
     }
@@ -1140,8 +1161,12 @@ int tqb_tq_cache_decode_fused(tqb_tq_cache* c, int32_t layer, const void* k, con
     if (dtype != TQB_F32 && dtype != TQB_F16 && dtype != TQB_BF16) return TQB_ERR_INVALID_ARGUMENT;
     if (!k || !v || !q || !out) return TQB_ERR_NULL_POINTER;
     cudaStream_t s = as_stream(stream);
-    TQB_TRY(c->store(layer, k, v, dtype, 1, s));
-    TQB_TRY(c->project(q, dtype, num_q_heads, 1, s));
+    int st = c->store_one_and_project(layer, k, v, q, dtype, num_q_heads, s);
+    if (st == TQB_ERR_UNSUPPORTED) {
+        TQB_TRY(c->store(layer, k, v, dtype, 1, s));
+        st = c->project(q, dtype, num_q_heads, 1, s);
+    }
+    if (st != TQB_OK) return st;
     auto* b = c->base;
     auto& L = b->layers[layer];
     tqb_decode_params p{};

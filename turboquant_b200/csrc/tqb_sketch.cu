@@ -351,6 +351,95 @@ projections_tile_kernel(const T* __restrict__ q, long long nq, const uint32_t* _
     }
 }
 
+// A decode step's input of the TQ cache.  The same work as block_quantize_pqo_kernel, block_dequantize_lane_kernel,
+// residual_sketch_kernel, a conversion and projections_kernel one after the other - the same operations in the same order, the
+// same bytes - for the few vectors of one token: a warp takes a head's K and V rows (a lane per 32-block quantizes, then the
+// warp dequantizes the key, sketches its residual), another warp takes a query.  What bounds it is the latency of
+// one chain: about 4 us, where the five launches took 17 us and as much again in the gaps between them.
+// Measured: 16 sequences x 4,001 tokens, 32 q / 8 KV heads, a layer's decode_fused call 76.6 -> 62 us.
+constexpr int kAppendWarps = 4;
+constexpr long long kAppendMax = 4096;   // keys and queries; about two rounds of the chip's warps, beyond which the separate kernels amortise their tables
+template <int W, typename T, int BITS>
+__global__ void __launch_bounds__(kAppendWarps * 32)
+tq_append_kernel(TqAppend a, const __grid_constant__ Codebook cb, float outer_centroid, float sign_mag, float inv_sqrt_d) {
+    constexpr int D = 32 * W;
+    __shared__ uint32_t s_rb[D * (W + 1)];
+    __shared__ float2 s_lut[kCells * 32];
+    __shared__ float s_vec[kAppendWarps][D];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    load_rbits<W>(s_rb, a.rbits);
+    build_cell_table(cb, cb.n - 1, s_lut, threadIdx.x, kAppendWarps * 32);
+    __syncthreads();
+    float* vec = s_vec[warp];
+    const long long item = (long long)blockIdx.x * kAppendWarps + warp;
+    if (item >= a.heads + a.nq) return;   // no block-wide barrier follows
+    if (item >= a.heads) {
+        const long long i = item - a.heads;
+#pragma unroll
+        for (int k = 0; k < W; ++k) vec[lane + 32 * k] = to_f32<T>(reinterpret_cast<const T*>(a.q)[i * D + lane + 32 * k]);
+        __syncwarp();
+        float proj[W];
+        rademacher_rows<W>(vec, s_rb, lane, inv_sqrt_d, proj);
+#pragma unroll
+        for (int k = 0; k < W; ++k) a.rq[i * D + lane + 32 * k] = proj[k];
+        return;
+    }
+    const T* key = reinterpret_cast<const T*>(a.k) + item * D;
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    uint16_t sc = 0;
+    if ((lane & 15) < W) {   // lanes 0 .. W-1: the key's blocks, 16 .. : the value's
+        const int b = lane & 15;
+        const T* src = (lane < 16 ? key : reinterpret_cast<const T*>(a.v) + item * D) + 32 * b;
+        sc = f32_to_f16_bits(pqo_quantize_block<T, BITS, true>(src, cb, outer_centroid, w, s_lut + lane));
+        const size_t blk = ((size_t)item * a.cap + a.row) * W + b;
+        uint32_t* out = reinterpret_cast<uint32_t*>((lane < 16 ? a.ki : a.vi) + blk * (4 * BITS));
+        out[0] = w[0]; out[1] = w[1]; out[2] = w[2];
+        if (BITS == 4) out[3] = w[3];
+        (lane < 16 ? a.ks : a.vs)[blk] = sc;
+    }
+    __syncwarp();
+    const float sgn = ((kSignMask >> lane) & 1u) ? -sign_mag : sign_mag, inv_sqrt = 1.0f / sqrtf((float)kBlock);
+    const int bit = BITS * lane, wi = bit >> 5;
+#pragma unroll
+    for (int b = 0; b < W; ++b) {
+        uint32_t kw[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) kw[i] = __shfl_sync(0xffffffffu, w[i], b);
+        const uint32_t lo = wi == 0 ? kw[0] : wi == 1 ? kw[1] : wi == 2 ? kw[2] : kw[3];
+        const uint32_t hi = wi == 0 ? kw[1] : wi == 1 ? kw[2] : kw[3];
+        const int code = min((int)(__funnelshift_r(lo, hi, bit & 31) & ((1u << BITS) - 1u)), cb.n - 1);
+        float y = cb.c[code] * sgn;
+#pragma unroll
+        for (int h = 1; h < 32; h <<= 1) {
+            const float other = __shfl_xor_sync(0xffffffffu, y, h);
+            y = (lane & h) ? (other - y) : (y + other);
+        }
+        y = (y * inv_sqrt) * fabsf(f16_bits_to_f32((uint16_t)__shfl_sync(0xffffffffu, (uint32_t)sc, b)));
+        vec[lane + 32 * b] = to_f32<T>(key[lane + 32 * b]) - y;
+    }
+    __syncwarp();
+    float s = 0.0f;   // left to right, every lane the same sum
+#pragma unroll 8
+    for (int c = 0; c < D; ++c) s = s + vec[c] * vec[c];
+    const size_t dst = (size_t)item * a.sketch_cap + a.row;
+    if (lane == 0) a.norms[dst] = f32_to_f16_bits(__fsqrt_rn(s));
+    float proj[W];
+    rademacher_rows<W>(vec, s_rb, lane, inv_sqrt_d, proj);
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+        const uint32_t word = __ballot_sync(0xffffffffu, proj[k] >= 0.0f);
+        if (lane == 0) reinterpret_cast<uint32_t*>(a.signs)[dst * W + k] = word;
+    }
+}
+
+template <int W, typename T>
+int launch_append(const TqAppend& a, const Codebook& cb, float outer, float sign_mag, float inv, cudaStream_t s) {
+    const long long grid = (a.heads + a.nq + kAppendWarps - 1) / kAppendWarps;
+    if (a.bits == 3) tq_append_kernel<W, T, 3><<<(unsigned)grid, kAppendWarps * 32, 0, s>>>(a, cb, outer, sign_mag, inv);
+    else tq_append_kernel<W, T, 4><<<(unsigned)grid, kAppendWarps * 32, 0, s>>>(a, cb, outer, sign_mag, inv);
+    return check_launch(s);
+}
+
 template <typename K>
 int opt_in(K kernel, size_t smem) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -428,6 +517,21 @@ int launch_projections_tile(int dim, const void* q, int dtype, long long nq, con
     if (dtype == TQB_F16) { TQB_PROJ(__half) }
     TQB_PROJ(__nv_bfloat16)
 #undef TQB_PROJ
+}
+
+int launch_tq_append(const TqAppend& a, cudaStream_t s) {
+    Codebook normal, outlier;
+    if ((a.bits != 3 && a.bits != 4) || !block_codebook(a.bits - 1, TQB_MAXNORM, normal) || !block_codebook(a.bits, TQB_MAXNORM, outlier))
+        return TQB_ERR_UNSUPPORTED;
+    const uintptr_t all = (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.q | (uintptr_t)a.ki | (uintptr_t)a.vi;
+    if ((all % 16) != 0 || ((uintptr_t)a.signs % 4) != 0 || a.heads + a.nq > kAppendMax) return TQB_ERR_UNSUPPORTED;
+    const float outer = outlier.c[outlier.n - 1];   // precomputed/mod.rs:78
+    volatile float inv32 = 1.0f / sqrtf(32.0f), s32 = sqrtf(32.0f);
+    const float sign_mag = inv32 * s32;             // src/cache/wht_tensor.rs:29-35: the sign pattern's magnitude in f32
+    const float inv = 1.0f / sqrtf((float)a.dim);
+    if (a.dtype == TQB_F32) { TQB_BY_DIM(a.dim, (launch_append<W, float>(a, normal, outer, sign_mag, inv, s))) }
+    if (a.dtype == TQB_F16) { TQB_BY_DIM(a.dim, (launch_append<W, __half>(a, normal, outer, sign_mag, inv, s))) }
+    TQB_BY_DIM(a.dim, (launch_append<W, __nv_bfloat16>(a, normal, outer, sign_mag, inv, s)))
 }
 
 }  // namespace tqb

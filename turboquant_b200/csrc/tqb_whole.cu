@@ -86,32 +86,6 @@ struct WholeArgs {
     float inv_sqrt_d;
 };
 
-// Sequential Rademacher row products of one vector held in shared memory.
-// Lane handles rows lane, lane+32, ...; s_rb has row stride W+1 words.
-template <int EPL>
-__device__ __forceinline__ void rademacher_rows(const float* vec, const uint32_t* s_rb, int lane, float inv_sqrt_d,
-                                                float (&proj)[EPL]) {
-    constexpr int W = EPL;
-    float s[EPL];
-#pragma unroll
-    for (int k = 0; k < EPL; ++k) s[k] = 0.0f;
-#pragma unroll 1
-    for (int cw = 0; cw < W; ++cw) {
-        uint32_t rb[EPL];
-#pragma unroll
-        for (int k = 0; k < EPL; ++k) rb[k] = s_rb[(lane + 32 * k) * (W + 1) + cw];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            const uint32_t val = __float_as_uint(vec[cw * 32 + c]);
-#pragma unroll
-            for (int k = 0; k < EPL; ++k)
-                s[k] = s[k] + __uint_as_float(val ^ ((rb[k] << (31 - c)) & 0x80000000u));
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < EPL; ++k) proj[k] = s[k] * inv_sqrt_d;
-}
-
 // quantize_vec (src/quantize.rs:142-192) and, with QJL outputs requested,
 // quantize_with_qjl (src/qjl.rs:355-377).  One warp per tile of 32 vectors.
 template <int EPL, bool QJL>
@@ -971,7 +945,7 @@ int grid_warps(long long n, int warps_per_block) {
 // From these batch sizes on the kernels of tqb_sketch.cu take over.  Quantize with sketch: two launches of about 19 us
 // against 8 us + 2.1 us a vector (128 dims: 16 vectors 19 against 41 us, 8 vectors 25 us sequentially).  Residual sketch and projections: below
 // 2,048 vectors one vector or query per warp fills the chip and takes 6 to 9 us; at 4,096 the tiles are ahead.
-constexpr long long kSketchMin = 16, kResidualTileMin = 2048, kProjTileMin = 2048;
+constexpr long long kSketchMin = 16, kResidualTileMin = 2048;   // (projections: kProjTileMin)
 
 float host_inv_sqrt(int dim) { return 1.0f / sqrtf((float)dim); }  // rotation.rs:36
 
