@@ -523,6 +523,60 @@ def test_pqo_cache_prefill_attend_two_chunks_then_decode(bits):
     assert dec.is_fused() and cache.seq_len(0) == 58 and torch.isfinite(dec.fused.float()).all()
 
 
+@pytest.mark.parametrize("bits,group,dtype", [(3, 4, torch.float32), (4, 8, torch.float32), (3, 7, torch.float32), (4, 1, torch.float32), (4, 4, torch.bfloat16)])
+@pytest.mark.parametrize("parts", [1, 2, 3, 7, 8, 9, 15, 16, 17, 24, 40])
+def test_merge_of_every_partition_count(bits, group, dtype, parts):
+    # one CTA, clusters of 2 .. 16, partials in the scratch merged in two levels: against the general kernel with one
+    # partition; most partitions are empty at 65 tokens
+    for kv_len in (65, 1999):
+        hkv, D = 3, 128
+        g = torch.Generator(device="cuda").manual_seed(kv_len + parts)
+        q = torch.randn((hkv * group, D), generator=g, device="cuda").to(dtype)
+        k, v = (torch.randn((hkv * kv_len, D), generator=g, device="cuda") for _ in range(2))
+        arrays = []
+        for t in (k, v):
+            i, s = tq.block_quantize(t, bits)
+            arrays += [i.view(hkv, kv_len, -1), s.view(hkv, kv_len, -1)]
+        want = tq.decode_attention(q, *arrays, kv_len, bits, 0.09, num_partitions=1, force_general=True, out_dtype=torch.float32)
+        got = tq.decode_attention(q, *arrays, kv_len, bits, 0.09, num_partitions=parts, out_dtype=torch.float32)
+        assert (got - want).abs().max().item() < TOL
+        out, lse = tq.decode_attention(q, *arrays, kv_len, bits, 0.09, num_partitions=parts, return_lse=True)
+        ref, rlse = tq.decode_attention(q, *arrays, kv_len, bits, 0.09, num_partitions=1, force_general=True, return_lse=True)
+        scale = torch.exp(lse[:, :1] - rlse[:, :1])       # the maxima may lie anywhere above the scores' own
+        assert ((out * scale - ref).abs().max() / ref.abs().max()).item() < TOL
+        assert ((lse[:, 1:] * scale - rlse[:, 1:]).abs() / rlse[:, 1:]).max().item() < TOL
+
+
+def test_ordered_launches_read_what_their_predecessor_wrote():
+    # each launch takes the previous launch's output as its query: a launch that starts early must not read it early
+    hkv, group, kv_len, D, bits = 8, 4, 700, 128, 3
+    g = torch.Generator(device="cuda").manual_seed(1)
+    arrays = []
+    for _ in range(2):
+        i, s = tq.block_quantize(torch.randn((hkv * kv_len, D), generator=g, device="cuda"), bits)
+        arrays += [i.view(hkv, kv_len, -1), s.view(hkv, kv_len, -1)]
+    cache = tq.PqoCache(tq.CacheConfig(bits=bits, head_dim=D, num_kv_heads=hkv, num_layers=2))
+    k = torch.randn((1, hkv, kv_len, D), generator=g, device="cuda")
+    for layer in range(2):
+        cache.prefill(layer, k, k)
+    att = tq.AttendConfig(0.09, group)
+    one = torch.randn((1, hkv, 1, D), generator=g, device="cuda")
+    q0 = torch.randn((1, hkv * group, 1, D), generator=g, device="cuda")
+    def chain(sync):
+        cache.reset()
+        for layer in range(2):
+            cache.prefill(layer, k, k)
+        q = q0
+        for step in range(40):
+            q = cache.decode(step % 2, one, one, q, att).fused * 20.0 if step % 3 == 0 else cache.decode(step % 2, one, one, q, att).fused
+            if sync:
+                torch.cuda.synchronize()
+        return q
+    want = chain(True)
+    for _ in range(5):
+        assert torch.equal(chain(False), want)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("bits,batch,hq,hkv,tokens", [(4, 1, 8, 2, (1, 129, 40)), (3, 3, 4, 4, (33, 31)), (4, 2, 16, 2, (17, 200)), (4, 2, 6, 2, (30, 5))])
 def test_prefill_attend_reads_queries_where_they_lie(bits, batch, hq, hkv, tokens, dtype):

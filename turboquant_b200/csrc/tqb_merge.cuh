@@ -112,134 +112,112 @@ __device__ __forceinline__ void merge_head(const MergeArgs& a, int head, int lan
     }
 }
 
-// The same merge for ALL g query heads of one KV head by one CTA of 128 threads, head_dim 128: thread d owns output
-// element d of every head (warp = 32-block, lane = element).  The slot weights exp(max_s - M) of all heads are
-// tabulated in shared memory, and each thread walks the slots eight at a time with the loads of all heads in flight
-// together, so a merge of S slots costs about S / 8 trips to L2 (merge_head makes one trip per slot, block and head).
+// The same merge for ALL g <= 8 query heads of one KV head by one CTA of 128 threads, head_dim 128: warp w owns heads w and
+// w + 4, lane = element of each of the four blocks.  All loads of a warp - up to eight slots of both heads and their
+// (max, sum) pairs - are in flight together, so a merge costs one trip to L2 and the arithmetic, and no warp waits for another.
+// (A thread per element going through all heads needs either 64 loads and as much code, which runs once and is fetched cold,
+// or a trip a head: 8 heads x 131,072 tokens in 74 partitions 70 or 75 us a launch.)
 //
 // Source: slots [first, first + count) of arrays laid out [head][head_stride][...] (a.partial_*).
 // Destination, GROUP = true: one more partial - un-normalised sum, max and sum of slot `gslot` of the group arrays
 // (a.group_*, [head][group_stride][...]), still in the rotated domain.  GROUP = false: the final result as merge_head
 // writes it (or, with num_copies > 0, the record copies).  Sums run over the slots in ascending order.
-// `s_work`: shared memory, at least (16 + g * count) floats; all 128 threads must call.
+// All 128 threads must call; there is no block-wide barrier inside.
 template <bool GROUP>
-__device__ __forceinline__ void merge_group128(const MergeArgs& a, int head0, int g, int tid, float* s_work, int first, int count,
-                                               int head_stride, int gslot = 0, int group_stride = 0) {
+__device__ __forceinline__ void merge_group128(const MergeArgs& a, int head0, int g, int tid, int first, int count, int head_stride,
+                                               int gslot = 0, int group_stride = 0) {
     using namespace merge_detail;
     const int lane = tid & 31, warp = tid >> 5;
     constexpr int D = 128;
-    float* s_M = s_work;          // [8]
-    float* s_L = s_work + 8;      // [8]
-    float* s_w = s_work + 16;     // [g][count]
-    // A dependent trip to L2 costs more than a microsecond on this part, so the loads of a merge are issued together:
-    // the first eight slots of the un-normalised outputs of all heads (up to 64 loads per thread) go out before the
-    // (max, sum) pairs are even looked at, and each warp fetches the pairs of both of its heads in one go.
-    const float* po = a.partial_out + ((size_t)head0 * head_stride + first) * D + tid;
-    float v[8][8];
-#pragma unroll
-    for (int hh = 0; hh < 8; ++hh)
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            v[hh][i] = (hh < g && i < count) ? __ldcg(po + ((size_t)hh * head_stride + i) * D) : 0.0f;
-    {
-        const float* pm[2];
-        const float* ps[2];
-        float pmv[2] = {-FLT_MAX, -FLT_MAX}, psv[2] = {0.0f, 0.0f};
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const int hh = warp + 4 * t;
-            pm[t] = a.partial_max + (size_t)(head0 + hh) * head_stride + first;
-            ps[t] = a.partial_sum + (size_t)(head0 + hh) * head_stride + first;
-            if (hh < g && lane < count) {
-                pmv[t] = __ldcg(pm[t] + lane);
-                psv[t] = __ldcg(ps[t] + lane);
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const int hh = warp + 4 * t;
-            if (hh >= g) continue;
-            float M = pmv[t];
-            for (int p = lane + 32; p < count; p += 32) M = fmaxf(M, __ldcg(pm[t] + p));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-            const float wl = lane < count ? expf(pmv[t] - M) : 0.0f;
-            if (lane < count) s_w[hh * count + lane] = wl;
-            float L = lane < count ? psv[t] * wl : 0.0f;
-            for (int p = lane + 32; p < count; p += 32) {
-                const float wp = expf(__ldcg(pm[t] + p) - M);
-                s_w[hh * count + p] = wp;
-                L += __ldcg(ps[t] + p) * wp;
-            }
-            L = sum32(L);
-            if (lane == 0) {
-                s_M[hh] = M;
-                s_L[hh] = L;
-            }
-        }
-    }
-    __syncthreads();
-    float acc[8];
-#pragma unroll
-    for (int hh = 0; hh < 8; ++hh) acc[hh] = 0.0f;
-    for (int p0 = 0; p0 < count; p0 += 8) {
-        if (p0 > 0) {
-#pragma unroll
-            for (int hh = 0; hh < 8; ++hh)
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    v[hh][i] = (hh < g && p0 + i < count) ? __ldcg(po + ((size_t)hh * head_stride + p0 + i) * D) : 0.0f;
-        }
-#pragma unroll
-        for (int hh = 0; hh < 8; ++hh)
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (hh < g && p0 + i < count) acc[hh] = fmaf(v[hh][i], s_w[hh * count + p0 + i], acc[hh]);
-    }
     const float inv_sqrt = 1.0f / sqrtf((float)kBlock);
     const uint32_t neg = 0xB1A6D4B2u;   // src/cache/precomputed/rotation.rs:16-20
     const float sg = a.dev_signs ? a.dev_signs[lane] : (((neg >> lane) & 1u) ? -a.sign_mag : a.sign_mag);
-    {
-        constexpr int h0 = 0;
+    float v[2][8][4], pm[2], pl[2];
 #pragma unroll
-        for (int hh = 0; hh < 8; ++hh) {
-            if (h0 + hh >= g) continue;
-            const int head = head0 + h0 + hh;
-            float r = acc[hh];
-            if (GROUP) {
-                a.group_out[((size_t)head * group_stride + gslot) * D + tid] = r;
-                continue;
-            }
-            if (a.rotate) r = wht32(r * sg, lane) * inv_sqrt;
-            if (a.num_copies > 0) {
-                // (constant indices only: a run-time index would move the argument block to local memory)
+    for (int t = 0; t < 2; ++t) {
+        const bool on = warp + 4 * t < g;
+        const size_t at = (size_t)(head0 + (on ? warp + 4 * t : 0)) * head_stride + first;
+        const float* po = a.partial_out + at * D + lane;
 #pragma unroll
-                for (int c = 0; c < kMaxPeers; ++c)
-                    if (c < a.num_copies) a.copy_rec[c][(size_t)head * D + tid] = r;
-                continue;
-            }
-            if (a.lse_out == nullptr) {
-                const float L = s_L[h0 + hh];
-                r *= L > 0.0f ? 1.0f / L : 0.0f;
-            }
-            store_out(a.out, a.out_dtype, (size_t)head * D + tid, r);
-        }
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) v[t][i][b] = (on && i < count) ? __ldcg(po + (size_t)i * D + 32 * b) : 0.0f;
+        pm[t] = (on && lane < count) ? __ldcg(a.partial_max + at + lane) : -FLT_MAX;
+        pl[t] = (on && lane < count) ? __ldcg(a.partial_sum + at + lane) : 0.0f;
     }
-    if (tid < g) {
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int head = head0 + warp + 4 * t;
+        if (warp + 4 * t >= g) break;
+        const size_t at = (size_t)head * head_stride + first;
+        float M = pm[t];
+        for (int p = lane + 32; p < count; p += 32) M = fmaxf(M, __ldcg(a.partial_max + at + p));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        const float wl = lane < count ? expf(pm[t] - M) : 0.0f;
+        float L = pl[t] * wl;
+        for (int p = lane + 32; p < count; p += 32) L += __ldcg(a.partial_sum + at + p) * expf(__ldcg(a.partial_max + at + p) - M);
+        L = sum32(L);
+        float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float w = __shfl_sync(0xffffffffu, wl, i);   // (0 past `count`)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) r[b] = fmaf(v[t][i][b], w, r[b]);
+        }
+#pragma unroll 1
+        for (int p0 = 8; p0 < count; p0 += 8) {
+            const float* po = a.partial_out + (at + p0) * D + lane;
+            float u[8][4];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) u[i][b] = p0 + i < count ? __ldcg(po + (size_t)i * D + 32 * b) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int p = p0 + i;
+                float w = __shfl_sync(0xffffffffu, wl, p & 31);
+                if (p >= 32) w = p < count ? expf(__ldcg(a.partial_max + at + p) - M) : 0.0f;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) r[b] = fmaf(u[i][b], w, r[b]);
+            }
+        }
         if (GROUP) {
-            a.group_max[(size_t)(head0 + tid) * group_stride + gslot] = s_M[tid];
-            a.group_sum[(size_t)(head0 + tid) * group_stride + gslot] = s_L[tid];
-        } else if (a.num_copies > 0) {
+            const size_t gi = (size_t)head * group_stride + gslot;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) a.group_out[gi * D + 32 * b + lane] = r[b];
+            if (lane == 0) {
+                a.group_max[gi] = M;
+                a.group_sum[gi] = L;
+            }
+            continue;
+        }
+        const float norm = (a.num_copies == 0 && a.lse_out == nullptr) ? (L > 0.0f ? 1.0f / L : 0.0f) : 1.0f;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            if (a.rotate) r[b] = wht32(r[b] * sg, lane) * inv_sqrt;
+            r[b] *= norm;
+        }
+        if (a.num_copies > 0) {
+            // (constant indices only: a run-time index would move the argument block to local memory)
 #pragma unroll
             for (int c = 0; c < kMaxPeers; ++c)
                 if (c < a.num_copies) {
-                    float* lse = a.copy_rec[c] + (size_t)a.num_q_heads * D;
-                    lse[(head0 + tid) * 2] = s_M[tid];
-                    lse[(head0 + tid) * 2 + 1] = s_L[tid];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) a.copy_rec[c][(size_t)head * D + 32 * b + lane] = r[b];
+                    if (lane == 0) {
+                        float* lse = a.copy_rec[c] + (size_t)a.num_q_heads * D;
+                        lse[head * 2] = M;
+                        lse[head * 2 + 1] = L;
+                    }
                 }
-        } else if (a.lse_out != nullptr) {
-            a.lse_out[(head0 + tid) * 2] = s_M[tid];
-            a.lse_out[(head0 + tid) * 2 + 1] = s_L[tid];
+            continue;
+        }
+#pragma unroll
+        for (int b = 0; b < 4; ++b) store_out(a.out, a.out_dtype, (size_t)head * D + 32 * b + lane, r[b]);
+        if (a.lse_out != nullptr && lane == 0) {
+            a.lse_out[head * 2] = M;
+            a.lse_out[head * 2 + 1] = L;
         }
     }
 }
