@@ -543,11 +543,16 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
     constexpr uint32_t kSD = TMA ? kWarps * 128 : 128;                  // from its K scale rows to its V scale rows
     const uint32_t ring = TMA ? rings_base + warp * G::kIdxB : rings_base + warp * G::kRingB;
     const uint32_t sdelta = TMA ? 2 * kWarps * G::kIdxB - warp * (G::kIdxB - 128) : 2 * G::kIdxB;   // K rows -> K scale rows
+    // kU groups of 16 tokens a step: their scores come before the one softmax of the step, their V products after it
+    // (with the sketch correction one: its words and digits leave no registers for a second group - 488 us a pass of
+    // 8 layers against 459 at 16 sequences x 4,001 tokens)
+    constexpr int kU = QJL ? 1 : 2, kAhead = kStages - kU;   // kAhead: stages in flight behind the ones being read
     FillPlan plan = TMA ? FillPlan{} : make_plan<BITS>(a, row0, first, lane);
     const uint32_t full0 = (uint32_t)__cvta_generic_to_shared(&s_bar[0][0]);
     const uint32_t empty0 = (uint32_t)__cvta_generic_to_shared(&s_bar[1][0]);
     const int ntiles = t_begin < t_end ? (t_end - t_begin + stride - 1) / stride : 0;   // 64-token tiles of the CTA
-    const int nsteps = TMA ? ntiles : ngroups;
+    // (the last step may hold a group past the end: it re-reads the last token and is masked)
+    const int nsteps = ((TMA ? ntiles : ngroups) + kU - 1) / kU * kU;
     const int trow0 = (int)row0 + t_begin;                     // TMA: token row of tile 0 in the whole array
     const bool producer = TMA && tid == 0;
     if (TMA) {
@@ -559,21 +564,21 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
             }
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 #pragma unroll
-            for (int i = 0; i < kStages - 1; ++i)
-                if (i < ntiles) tma_tile_fill<BITS>(maps, rings_base + i * G::kTileB, full0 + 8 * i, trow0 + i * stride);
+            for (int i = 0; i < kAhead; ++i)
+                if (i < nsteps) tma_tile_fill<BITS>(maps, rings_base + i * G::kTileB, full0 + 8 * i, trow0 + i * stride);
         }
         // the other threads first touch a barrier after the block-wide barriers of the query prologue
     } else {
 #pragma unroll
-        for (int i = 0; i < kStages - 1; ++i) {
-            stage_fill<BITS>(plan, i < ngroups, first + i * stride + kGroup > last + 1, stride, first + i * stride, last, ring + i * G::kStageB);
+        for (int i = 0; i < kAhead; ++i) {
+            stage_fill<BITS>(plan, i < nsteps, first + i * stride + kGroup > last + 1, stride, first + i * stride, last, ring + i * G::kStageB);
             cp_async_commit();
         }
     }
     uint32_t st = ring;                                        // stage being consumed (this warp's K rows)
-    uint32_t st_fill = TMA ? rings_base + (kStages - 1) * G::kTileB : ring + (kStages - 1) * G::kStageB;   // stage being refilled
+    uint32_t st_fill = TMA ? rings_base + kAhead * G::kTileB : ring + kAhead * G::kStageB;   // stage being refilled
     // TMA: barrier offset (8 x stage) of st / of st_fill, phase of st's full barrier, phase of st_fill's empty barrier
-    uint32_t boff = 0, boff_fill = 8 * (kStages - 1), parity = 0, eparity = 1;
+    uint32_t boff = 0, boff_fill = 8 * kAhead, parity = 0, eparity = 1;
     bool stage_ok = true;
 
     // per-thread shared-memory offsets inside a stage; every load of the token loop is one of three or four
@@ -763,10 +768,9 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
         rqc[e] = QJL ? s_qsc[NSPLIT ? j : 2 * j + e] * a.qjl_const : 0.0f;
         rqsum[e] = QJL ? s_rqsum[NSPLIT ? j : 2 * j + e] : 0;
     }
-    // QJL: sketch word j and residual norm of tokens n and n + 8 of the step, fetched two steps ahead (tokens past
-    // the end re-read the last token; they are masked later)
-    uint32_t sgw[2] = {0u, 0u};
-    uint32_t nrw[2] = {0u, 0u};
+    // QJL: sketch word j and residual norm of tokens n and n + 8, fetched two groups ahead - one is shorter than a trip to
+    // HBM (tokens past the end re-read the last token; they are masked later)
+    uint32_t sgw[2][2], nrw[2][2];   // this group, the next
     auto qjl_fetch = [&](int it, uint32_t (&sg)[2], uint32_t (&nr)[2]) {
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
@@ -775,11 +779,11 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
             nr[t] = __ldg(a.qjl_norms + row);
         }
     };
-    // (two steps ahead: one step is shorter than a trip to HBM)
-    uint32_t sg1[2] = {0u, 0u};
-    uint32_t nr1[2] = {0u, 0u};
-    if (QJL && nsteps > 0) qjl_fetch(0, sgw, nrw);
-    if (QJL && nsteps > 1) qjl_fetch(1, sg1, nr1);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        sgw[u][0] = sgw[u][1] = nrw[u][0] = nrw[u][1] = 0u;
+        if (QJL && u < nsteps) qjl_fetch(u, sgw[u], nrw[u]);
+    }
     float m_run[kE], l_run[kE];   // per head; l_run: this lane's tokens only
 #pragma unroll
     for (int e = 0; e < kE; ++e) {
@@ -796,35 +800,53 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
 
     // Loop control in terms of iteration numbers fixed before the loop: the last step that still refills a
     // stage, the step whose refill is the (only possibly) ragged last group, and the first step with tokens to mask.
-    const int fill_end = ngroups - (kStages - 1);                                    // refill while it < fill_end
-    const int rag_fill_it = (first + (ngroups - 1) * stride + kGroup > last + 1) ? fill_end - 1 : -1;
+    const int rag_fill = (last + 1 - kGroup - first < 0) ? 0 : (last + 1 - kGroup - first) / stride + 1;   // the first group that runs past the last token
     const int rag_from = (t_end - kGroup - first < 0) ? 0 : (t_end - kGroup - first) / stride + 1;
-    uint32_t st_prev = ring + (kStages - 1) * kPitch;   // cp.async: the stage consumed one step ago is the one refilled now
-#pragma unroll 2
-    for (int it = 0; it < nsteps; ++it) {
+    for (int it = 0; it < nsteps; it += kU) {
+        uint32_t stu[kU];   // the stages of the step's groups
         if (TMA) {
             // A warp whose 16 rows of the tile lie past the end of the partition runs the step on them all
             // the same: every such token is masked below and contributes exactly nothing.
-            if (producer && it + kStages - 1 < ntiles) {
-                // refill the stage of tile it - 1 once all four warps have released it
-                if (it >= 1 && !mbar_wait(empty0 + boff_fill, eparity)) stage_ok = false;
-                else tma_tile_fill<BITS>(maps, st_fill, full0 + boff_fill, trow0 + (it + kStages - 1) * stride);
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                if (producer && it + kAhead + u < nsteps) {
+                    // refill the stage of tile it + u - kU once all four warps have released it
+                    if (it >= kU && !mbar_wait(empty0 + boff_fill, eparity)) stage_ok = false;
+                    else tma_tile_fill<BITS>(maps, st_fill, full0 + boff_fill, trow0 + (it + kAhead + u) * stride);
+                }
+                __syncwarp();
+                if (boff_fill + 8 == 8 * kStages) { boff_fill = 0; eparity ^= 1u; } else boff_fill += 8;
+                st_fill = (st_fill + kPitch == rings_base + kStages * kPitch) ? rings_base : st_fill + kPitch;
             }
-            __syncwarp();
-            if (boff_fill + 8 == 8 * kStages) { boff_fill = 0; eparity ^= 1u; } else boff_fill += 8;
-            st_fill = (st_fill + kPitch == rings_base + kStages * kPitch) ? rings_base : st_fill + kPitch;
-            if (!mbar_wait(full0 + boff, parity)) {   // never expected: give up on this partition and say so
+            bool landed = true;
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                landed = landed && mbar_wait(full0 + boff, parity);
+                if (boff + 8 == 8 * kStages) { boff = 0; parity ^= 1u; } else boff += 8;
+            }
+            if (!landed) {   // never expected: give up on this partition and say so
                 stage_ok = false;
                 break;
             }
         } else {
-            stage_fill<BITS>(plan, it < fill_end, it == rag_fill_it, stride, first + (it + kStages - 1) * stride, last, st_prev);
-            cp_async_commit();
-            cp_async_wait<kStages - 1>();
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                stage_fill<BITS>(plan, it + kAhead + u < nsteps, it + kAhead + u >= rag_fill, stride, first + (it + kAhead + u) * stride, last, st_fill);
+                cp_async_commit();
+                st_fill = (st_fill + kPitch == ring + kStages * kPitch) ? ring : st_fill + kPitch;
+            }
+            cp_async_wait<kAhead>();
             __syncwarp();
         }
-
-        const uint32_t bK0 = st + offK0, bK1 = st + offK1, bS = st + offS;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            stu[u] = st;
+            st = (st + kPitch == ring + kStages * kPitch) ? ring : st + kPitch;
+        }
+        float sc[kU][2][kE];   // scores [group][token n | n + 8][head]
+        static_for<0, kU>([&](auto u_) {
+        constexpr int u = decltype(u_)::value;
+        const uint32_t bK0 = stu[u] + offK0, bK1 = stu[u] + offK1, bS = stu[u] + offS;
         // ---- S = K~ Q~^T : rows = tokens (n, n + 8), columns = heads ----
         uint32_t kw[2][4];   // 4-bit: [block pair][octet | block parity << 1] -> word j of token n of the octet
         if (BITS == 4) {
@@ -898,20 +920,20 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
                 }
             });
         }
-        float sc[2][kE];   // scores [token n | n + 8][head]
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
-            for (int e = 0; e < kE; ++e) sc[t][e] = BITS == 4 ? s[t][e] * qsc[e] : s[t][e];
+            for (int e = 0; e < kE; ++e) sc[u][t][e] = BITS == 4 ? s[t][e] * qsc[e] : s[t][e];
         if constexpr (QJL) {
+            static_assert(kU == 1, "the sketch words are passed on group by group");
             uint32_t sgn[2] = {0u, 0u}, nrn[2] = {0u, 0u};
-            if (it + 2 < nsteps) qjl_fetch(it + 2, sgn, nrn);   // the sketch words of the step after next, in flight for two steps
+            if (it + 2 < nsteps) qjl_fetch(it + 2, sgn, nrn);
             int ca[4] = {0, 0, 0, 0}, cb[4] = {0, 0, 0, 0}, cc[4] = {0, 0, 0, 0};
             static_for<0, 4>([&](auto m_) {
                 constexpr int m4 = decltype(m_)::value;
                 // bytes i of the four operands: sign bits 2 m4 + 8 i (and 2 m4 + 1 + 8 i) of the two tokens' words
-                const uint32_t a0 = (sgw[0] >> (2 * m4)) & 0x01010101u, a1 = (sgw[1] >> (2 * m4)) & 0x01010101u;
-                const uint32_t a2 = (sgw[0] >> (2 * m4 + 1)) & 0x01010101u, a3 = (sgw[1] >> (2 * m4 + 1)) & 0x01010101u;
+                const uint32_t a0 = (sgw[0][0] >> (2 * m4)) & 0x01010101u, a1 = (sgw[0][1] >> (2 * m4)) & 0x01010101u;
+                const uint32_t a2 = (sgw[0][0] >> (2 * m4 + 1)) & 0x01010101u, a3 = (sgw[0][1] >> (2 * m4 + 1)) & 0x01010101u;
                 const uint4 r4 = lds128_volatile_o<m4 * 512>(rqfr_base);
                 imma16832_acc(ca, a0, a1, a2, a3, r4.x, r4.y);
                 imma16832_acc(cb, a0, a1, a2, a3, r4.z, r4.w);
@@ -920,52 +942,55 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
                     imma16832_acc(cc, a0, a1, a2, a3, r2.x, r2.y);
                 }
             });
-            const float n0 = __half2float(__ushort_as_half((unsigned short)nrw[0]));
-            const float n1 = __half2float(__ushort_as_half((unsigned short)nrw[1]));
+            const float n0 = __half2float(__ushort_as_half((unsigned short)nrw[0][0]));
+            const float n1 = __half2float(__ushort_as_half((unsigned short)nrw[0][1]));
             if (NSPLIT) {   // ca: columns (D2, D1) of head j, cb: (D0, -)
                 const int i0 = (int)((uint32_t)ca[0] * 65536u + (uint32_t)ca[1] * 256u + (uint32_t)cb[0]);
                 const int i1 = (int)((uint32_t)ca[2] * 65536u + (uint32_t)ca[3] * 256u + (uint32_t)cb[2]);
-                sc[0][0] = fmaf((float)(2 * i0 - rqsum[0]), n0 * rqc[0], sc[0][0]);
-                sc[1][0] = fmaf((float)(2 * i1 - rqsum[0]), n1 * rqc[0], sc[1][0]);
+                sc[u][0][0] = fmaf((float)(2 * i0 - rqsum[0]), n0 * rqc[0], sc[u][0][0]);
+                sc[u][1][0] = fmaf((float)(2 * i1 - rqsum[0]), n1 * rqc[0], sc[u][1][0]);
             } else {        // ca / cb / cc: digits D2 / D1 / D0 of heads 2j, 2j+1
                 int iv[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) iv[i] = (int)((uint32_t)ca[i] * 65536u + (uint32_t)cb[i] * 256u + (uint32_t)cc[i]);
-                sc[0][0] = fmaf((float)(2 * iv[0] - rqsum[0]), n0 * rqc[0], sc[0][0]);
-                sc[0][1] = fmaf((float)(2 * iv[1] - rqsum[1]), n0 * rqc[1], sc[0][1]);
-                sc[1][0] = fmaf((float)(2 * iv[2] - rqsum[0]), n1 * rqc[0], sc[1][0]);
-                sc[1][1] = fmaf((float)(2 * iv[3] - rqsum[1]), n1 * rqc[1], sc[1][1]);
+                sc[u][0][0] = fmaf((float)(2 * iv[0] - rqsum[0]), n0 * rqc[0], sc[u][0][0]);
+                sc[u][0][1] = fmaf((float)(2 * iv[1] - rqsum[1]), n0 * rqc[1], sc[u][0][1]);
+                sc[u][1][0] = fmaf((float)(2 * iv[2] - rqsum[0]), n1 * rqc[0], sc[u][1][0]);
+                sc[u][1][1] = fmaf((float)(2 * iv[3] - rqsum[1]), n1 * rqc[1], sc[u][1][1]);
             }
-            sgw[0] = sg1[0]; sgw[1] = sg1[1]; nrw[0] = nr1[0]; nrw[1] = nr1[1];
-            sg1[0] = sgn[0]; sg1[1] = sgn[1]; nr1[0] = nrn[0]; nr1[1] = nrn[1];
+            sgw[0][0] = sgw[1][0]; sgw[0][1] = sgw[1][1]; nrw[0][0] = nrw[1][0]; nrw[0][1] = nrw[1][1];
+            sgw[1][0] = sgn[0]; sgw[1][1] = sgn[1]; nrw[1][0] = nrn[0]; nrw[1][1] = nrn[1];
         }
-        if (it >= rag_from) {   // ragged tail: tokens past the end (of the sequence, or of the partition) get zero weight
-            const int gs = first + it * stride;
+        if (it + u >= rag_from) {   // ragged tail: tokens past the end (of the sequence, or of the partition) get zero weight
+            const int gs = first + (it + u) * stride;
             if (TMA) {
                 // the tensor copies brought whatever lies behind the last token: clear those scale rows, so
                 // that a zero probability never meets an Inf or NaN scale
                 const int t = lane & 15;
                 if (gs + t >= t_end)
-                    asm volatile("st.shared.v2.u32 [%0], {%1, %1};\n" ::"r"(st + sdelta + (lane >> 4) * kSD + t * 8), "r"(0u) : "memory");
+                    asm volatile("st.shared.v2.u32 [%0], {%1, %1};\n" ::"r"(stu[u] + sdelta + (lane >> 4) * kSD + t * 8), "r"(0u) : "memory");
                 __syncwarp();
             }
 #pragma unroll
             for (int t = 0; t < 2; ++t)
                 if (gs + n + 8 * t >= t_end) {
 #pragma unroll
-                    for (int e = 0; e < kE; ++e) sc[t][e] = kNegBig;
+                    for (int e = 0; e < kE; ++e) sc[u][t][e] = kNegBig;
                 }
         }
-        // ---- online softmax: the 16 tokens of a head are spread over the 8 lane groups n ----
+        });
+        // ---- online softmax: the step's tokens of a head are spread over the 8 lane groups n ----
         // The reference value m_run is only raised when the step's maximum exceeds it by more than kLazy
         // (in log2 units): any common reference gives the same result, p stays below 2^kLazy, and the
         // rescaling of the 32 accumulators becomes rare.
         constexpr float kLazy = 6.0f;
-        float resc[kE], p[2][kE];
+        float resc[kE], p[kU][2][kE];
         bool changed = false;
 #pragma unroll
         for (int e = 0; e < kE; ++e) {
-            float mx = fmaxf(sc[0][e], sc[1][e]);
+            float mx = fmaxf(sc[0][0][e], sc[0][1][e]);
+#pragma unroll
+            for (int u = 1; u < kU; ++u) mx = fmaxf(mx, fmaxf(sc[u][0][e], sc[u][1][e]));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
@@ -973,9 +998,14 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
             resc[e] = ex2(m_run[e] - m_new);
             changed |= resc[e] != 1.0f;
             m_run[e] = m_new;
-            p[0][e] = ex2(sc[0][e] - m_new);
-            p[1][e] = ex2(sc[1][e] - m_new);
-            l_run[e] = l_run[e] * resc[e] + (p[0][e] + p[1][e]);
+            float add = 0.0f;
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                p[u][0][e] = ex2(sc[u][0][e] - m_new);
+                p[u][1][e] = ex2(sc[u][1][e] - m_new);
+                add += p[u][0][e] + p[u][1][e];
+            }
+            l_run[e] = l_run[e] * resc[e] + add;
         }
         if (__any_sync(0xffffffffu, changed)) {
             // columns (2j, 2j+1) of O^T: NSPLIT the hi and lo column of head j, otherwise heads 2j and 2j+1
@@ -993,11 +1023,14 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
         // relative.  movmatrix takes registers holding the lane's two columns of one token row - NSPLIT: (hi, lo)
         // of head j, otherwise the hi (or lo) parts of heads 2j, 2j+1 - and turns each 8 x 8 matrix (token rows,
         // columns) into the B fragment (tokens 2j, 2j+1 of column n) of O^T = V^T P'.
+        static_for<0, kU>([&](auto u_) {
+        constexpr int u = decltype(u_)::value;
+        const uint32_t bK0 = stu[u] + offK0, bK1 = stu[u] + offK1, bS = stu[u] + offS;
         uint32_t pq[NSPLIT ? 1 : 2][4][2];   // [hi | lo][block][octet]
         if (NSPLIT) {
             // one head per lane: the half2 lanes run over the two tokens (n, n + 8); three instructions per
             // block give (hi', hi') and (lo', lo') of both tokens, two PRMTs re-pair them per token
-            const __half2 ph = u32_as_h2(pack_hi(p[0][0], p[1][0])), pl = u32_as_h2(pack_lo(p[0][0], p[1][0]));
+            const __half2 ph = u32_as_h2(pack_hi(p[u][0][0], p[u][1][0])), pl = u32_as_h2(pack_lo(p[u][0][0], p[u][1][0]));
             const uint2 vs0 = lds64_o<kSD>(bS), vs1 = lds64_o<kSD + 64>(bS);   // V scale rows of tokens n, n + 8
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
@@ -1010,8 +1043,8 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
         } else {
             static_for<0, 2>([&](auto t_) {
                 constexpr int t = decltype(t_)::value;
-                const __half2 ph = u32_as_h2(pack_hi(p[t][0], p[t][kE - 1]));
-                const __half2 pl = u32_as_h2(pack_lo(p[t][0], p[t][kE - 1]));
+                const __half2 ph = u32_as_h2(pack_hi(p[u][t][0], p[u][t][kE - 1]));
+                const __half2 pl = u32_as_h2(pack_lo(p[u][t][0], p[u][t][kE - 1]));
                 const uint2 vsr = lds64_o<kSD + t * 64>(bS);   // V scale row of token n + 8t
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
@@ -1030,7 +1063,7 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
             ldsm4t_o<kVD>(bK0, vw[0]);
             ldsm4t_o<kVD>(bK1, vw[1]);
         }
-        const uint32_t bV = st + offV, bVh = st + offVh;   // 3-bit only
+        const uint32_t bV = stu[u] + offV, bVh = stu[u] + offVh;   // 3-bit only
         static_for<0, 4>([&](auto b_) {
             constexpr int b = decltype(b_)::value;
             // codes 4n..4n+3 of block b of the four tokens, paired (token 2j, token 2j+1)
@@ -1060,12 +1093,12 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
                 mma16816(o[b][1], xab[2], xab[3], xcd[2], xcd[3], pq[ps][b][0], pq[ps][b][1]);
             }
         });
-        __syncwarp();   // every lane is done with this stage before it is refilled
-        st_prev = st;
-        st = (st + kPitch == ring + kStages * kPitch) ? ring : st + kPitch;
+        });
+        __syncwarp();   // every lane is done with these stages before they are refilled
         if (TMA) {
-            if (lane == 0) mbar_arrive(empty0 + boff);   // this warp releases its rows of the tile
-            if (boff + 8 == 8 * kStages) { boff = 0; parity ^= 1u; } else boff += 8;
+#pragma unroll
+            for (int u = 0; u < kU; ++u)
+                if (lane == 0) mbar_arrive(empty0 + (stu[u] - ring) / kPitch * 8);   // this warp releases its rows of the tile
         }
     }
     bool gave_up = false;
