@@ -692,6 +692,32 @@ struct tqb_kv_cache {
     std::vector<Layer> layers;
     uint32_t* rbits = nullptr;
     DevBuf stage_a, stage_b, wv_scratch;
+    // Calls on short lists exchange a few kilobytes with the kernels through one page of mapped host memory: a pageable
+    // copy costs the host 10 us each way and stands between the launch and its result.
+    static constexpr size_t kMappedFloats = 4096;
+    float *mapped = nullptr, *mapped_dev = nullptr;
+    unsigned* ticket = nullptr;
+    bool map_tried = false;
+
+    bool small_calls(int64_t n) {
+        if (n > (int64_t)kMappedFloats - 256) return false;
+        if (!map_tried) {
+            map_tried = true;
+            if (cudaHostAlloc((void**)&mapped, kMappedFloats * sizeof(float), cudaHostAllocMapped) != cudaSuccess ||
+                cudaHostGetDevicePointer((void**)&mapped_dev, mapped, 0) != cudaSuccess ||
+                cudaMalloc((void**)&ticket, 256) != cudaSuccess || cudaMemset(ticket, 0, 256) != cudaSuccess) {
+                cudaGetLastError();
+                release_small();
+            }
+        }
+        return ticket != nullptr;
+    }
+    void release_small() {
+        if (mapped) cudaFreeHost(mapped);
+        if (ticket) cudaFree(ticket);
+        mapped = mapped_dev = nullptr;
+        ticket = nullptr;
+    }
 
     void free_side(Side& s) {
         if (s.packed) cudaFree(s.packed);
@@ -771,6 +797,7 @@ void tqb_kv_cache_destroy(tqb_kv_cache* c) {
         c->free_side(l.v);
     }
     if (c->rbits) cudaFree(c->rbits);
+    c->release_small();
     c->stage_a.release(); c->stage_b.release(); c->wv_scratch.release();
     delete c;
 }
@@ -818,6 +845,15 @@ int tqb_kv_cache_attention_scores(tqb_kv_cache* c, int32_t layer, const float* q
     if (!query || !scores) return TQB_ERR_NULL_POINTER;
     cudaStream_t s = as_stream(stream);
     const int d = c->cfg.dim;
+    if (c->small_calls(L.nk)) {
+        const int st = launch_scores_query(&c->cfg, c->rbits, query, L.k.packed, L.k.scales, L.k.signs, L.k.rnorms, L.nk, c->mapped_dev, s);
+        if (st == TQB_OK) {
+            TQB_CUDA(cudaStreamSynchronize(s));
+            std::memcpy(scores, c->mapped, (size_t)L.nk * sizeof(float));
+            return TQB_OK;
+        }
+        if (st != TQB_ERR_UNSUPPORTED) return st;
+    }
     TQB_TRY(c->stage_a.reserve(std::max<size_t>(2 * d * sizeof(float), c->stage_a.bytes)));
     TQB_TRY(c->stage_b.reserve((size_t)L.nk * sizeof(float)));
     float* qd = (float*)c->stage_a.p;
@@ -846,6 +882,18 @@ int tqb_kv_cache_weighted_values(tqb_kv_cache* c, int32_t layer, const float* we
         return TQB_OK;
     }
     if (!weights) return TQB_ERR_NULL_POINTER;
+    if (c->small_calls(n)) {
+        TQB_TRY(c->wv_scratch.reserve(tqb_weighted_values_scratch_bytes(d)));
+        std::memcpy(c->mapped + 256, weights, (size_t)n * sizeof(float));   // (nothing is in flight: every call ends synchronised)
+        const int st = launch_weighted_values_one(&c->cfg, c->mapped_dev + 256, L.v.packed, L.v.scales, n, c->mapped_dev,
+                                                  (float*)c->wv_scratch.p, c->ticket, s);
+        if (st == TQB_OK) {
+            TQB_CUDA(cudaStreamSynchronize(s));
+            std::memcpy(out, c->mapped, sizeof(float) * d);
+            return TQB_OK;
+        }
+        if (st != TQB_ERR_UNSUPPORTED) return st;
+    }
     TQB_TRY(c->stage_a.reserve((size_t)n * sizeof(float)));
     TQB_TRY(c->stage_b.reserve((size_t)d * sizeof(float)));
     TQB_TRY(c->wv_scratch.reserve(tqb_weighted_values_scratch_bytes(d)));

@@ -62,4 +62,11 @@ struct TqAppend {
 };
 int launch_tq_append(const TqAppend& a, cudaStream_t s);
 
+// QuantizedKVCache on short lists (tqb_whole.cu): one launch, host-mapped results.
+int launch_scores_query(const tqb_config* cfg, const uint32_t* rbits, const float* q_host, const uint8_t* packed,
+                        const uint16_t* scales, const uint8_t* signs, const uint16_t* rnorms, long long n, float* scores,
+                        cudaStream_t s);
+int launch_weighted_values_one(const tqb_config* cfg, const float* w, const uint8_t* packed, const uint16_t* scales, long long n,
+                               float* out, float* partial, unsigned* ticket, cudaStream_t s);
+
 }  // namespace tqb

@@ -503,22 +503,12 @@ __device__ __forceinline__ float warp_sum(float v) {
 // attention_scores (src/attention.rs:319-353, src/qjl.rs:585-606).  The key is never
 // rotated back: <q, s * sigma .* H(c)/sqrt(d)> = s * <H(sigma .* q)/sqrt(d), c>.
 template <int EPL>
-__global__ void scores_kernel(const float* __restrict__ q, const float* __restrict__ rq,
-                              const uint8_t* __restrict__ packed, const uint16_t* __restrict__ scales,
-                              const uint8_t* __restrict__ signs, const uint16_t* __restrict__ rnorms, long long n,
-                              float* __restrict__ scores, Codebook cb, int bits, int pb, uint64_t seed,
-                              float inv_sqrt_d, float sqrt_d) {
+__device__ __forceinline__ void scores_body(float (&qr)[EPL], const float (&rqv)[EPL], const float* s_c,
+                                            const uint8_t* __restrict__ packed, const uint16_t* __restrict__ scales,
+                                            const uint8_t* __restrict__ signs, const uint16_t* __restrict__ rnorms, long long n,
+                                            float* __restrict__ scores, int bits, int pb, float inv_sqrt_d, float sqrt_d) {
     constexpr int D = 32 * EPL, W = EPL;
-    __shared__ float s_c[16];
-    if (threadIdx.x < 16) s_c[threadIdx.x] = cb.c[threadIdx.x];
-    __syncthreads();
     const int lane = threadIdx.x & 31;
-    float qr[EPL], rqv[EPL];
-#pragma unroll
-    for (int k = 0; k < EPL; ++k) {
-        qr[k] = q[lane + 32 * k] * sign_of(seed, lane + 32 * k);
-        rqv[k] = rq[lane + 32 * k];
-    }
     wht_lanes<EPL>(qr, lane);
 #pragma unroll
     for (int k = 0; k < EPL; ++k) qr[k] = qr[k] * inv_sqrt_d;
@@ -564,15 +554,109 @@ __global__ void scores_kernel(const float* __restrict__ q, const float* __restri
     }
 }
 
+template <int EPL>
+__global__ void scores_kernel(const float* __restrict__ q, const float* __restrict__ rq,
+                              const uint8_t* __restrict__ packed, const uint16_t* __restrict__ scales,
+                              const uint8_t* __restrict__ signs, const uint16_t* __restrict__ rnorms, long long n,
+                              float* __restrict__ scores, Codebook cb, int bits, int pb, uint64_t seed,
+                              float inv_sqrt_d, float sqrt_d) {
+    __shared__ float s_c[16];
+    if (threadIdx.x < 16) s_c[threadIdx.x] = cb.c[threadIdx.x];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    float qr[EPL], rqv[EPL];
+#pragma unroll
+    for (int k = 0; k < EPL; ++k) {
+        qr[k] = q[lane + 32 * k] * sign_of(seed, lane + 32 * k);
+        rqv[k] = rq[lane + 32 * k];
+    }
+    scores_body<EPL>(qr, rqv, s_c, packed, scales, signs, rnorms, n, scores, bits, pb, inv_sqrt_d, sqrt_d);
+}
+
+// The same for one query that comes as a kernel argument: every CTA projects it itself (thread r adds row r left to right, as
+// projections_kernel does), so a call on host data is one launch and no copy of the query.
+struct QueryArg {
+    float q[256];
+};
+template <int EPL>
+__global__ void __launch_bounds__(256)
+scores_query_kernel(const __grid_constant__ QueryArg query, const uint32_t* __restrict__ rbits,
+                    const uint8_t* __restrict__ packed, const uint16_t* __restrict__ scales,
+                    const uint8_t* __restrict__ signs, const uint16_t* __restrict__ rnorms, long long n,
+                    float* __restrict__ scores, const __grid_constant__ Codebook cb, int bits, int pb, uint64_t seed,
+                    float inv_sqrt_d, float sqrt_d) {
+    constexpr int D = 32 * EPL, W = EPL;
+    __shared__ float s_c[16], s_rq[D];
+    if (threadIdx.x < 16) s_c[threadIdx.x] = cb.c[threadIdx.x];
+    if (threadIdx.x < D) {
+        float s = 0.0f;
+#pragma unroll
+        for (int cw = 0; cw < W; ++cw) {
+            const uint32_t word = __ldg(rbits + threadIdx.x * W + cw);
+#pragma unroll
+            for (int c = 0; c < 32; ++c)
+                s = s + __uint_as_float(__float_as_uint(query.q[cw * 32 + c]) ^ ((word << (31 - c)) & 0x80000000u));
+        }
+        s_rq[threadIdx.x] = s * inv_sqrt_d;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    float qr[EPL], rqv[EPL];
+#pragma unroll
+    for (int k = 0; k < EPL; ++k) {
+        qr[k] = query.q[lane + 32 * k] * sign_of(seed, lane + 32 * k);
+        rqv[k] = s_rq[lane + 32 * k];
+    }
+    scores_body<EPL>(qr, rqv, s_c, packed, scales, signs, rnorms, n, scores, bits, pb, inv_sqrt_d, sqrt_d);
+}
+
 constexpr int kWvBlocks = 296;  // two CTAs per SM
 constexpr long long kListMin = 4096;   // shorter lists stay on the warp-per-key kernels (no table build)
+
+// 256 threads
+template <int EPL>
+__device__ __forceinline__ void weighted_values_final(const float* partial, int nparts, float* __restrict__ out, uint64_t seed,
+                                                      float inv_sqrt_d, float (*s_part)[32 * EPL]) {
+    constexpr int D = 32 * EPL;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float v[EPL];
+#pragma unroll
+    for (int k = 0; k < EPL; ++k) v[k] = 0.0f;
+    for (int p = warp; p < nparts; p += 8) {
+#pragma unroll
+        for (int k = 0; k < EPL; ++k) v[k] += __ldcg(partial + (size_t)p * D + lane + 32 * k);
+    }
+#pragma unroll
+    for (int k = 0; k < EPL; ++k) s_part[warp][lane + 32 * k] = v[k];
+    __syncthreads();
+    if (warp != 0) return;
+#pragma unroll
+    for (int k = 0; k < EPL; ++k) {
+        float s = 0.0f;
+#pragma unroll
+        for (int ww = 0; ww < 8; ++ww) s += s_part[ww][lane + 32 * k];
+        v[k] = s;
+    }
+    wht_lanes<EPL>(v, lane);
+#pragma unroll
+    for (int k = 0; k < EPL; ++k) out[lane + 32 * k] = (v[k] * inv_sqrt_d) * sign_of(seed, lane + 32 * k);
+}
+
+template <int EPL>
+__global__ void __launch_bounds__(256)
+weighted_values_final_kernel(const float* __restrict__ partial, int nparts, float* __restrict__ out, uint64_t seed,
+                             float inv_sqrt_d) {
+    __shared__ float s_part[8][32 * EPL];
+    weighted_values_final<EPL>(partial, nparts, out, seed, inv_sqrt_d, s_part);
+}
 
 // weighted_values (src/attention.rs:371-408), accumulated in the rotated domain:
 // sum_t w_t s_t sigma .* H(c_t)/sqrt(d) = sigma .* H(sum_t w_t s_t c_t)/sqrt(d).
 template <int EPL>
 __global__ void weighted_values_partial_kernel(const float* __restrict__ w, const uint8_t* __restrict__ packed,
                                                const uint16_t* __restrict__ scales, long long n,
-                                               float* __restrict__ partial, Codebook cb, int bits, int pb) {
+                                               float* __restrict__ partial, Codebook cb, int bits, int pb, unsigned* ticket,
+                                               float* __restrict__ out, uint64_t seed, float inv_sqrt_d) {
     constexpr int D = 32 * EPL;
     __shared__ float s_c[16];
     __shared__ float s_acc[8][D];
@@ -609,36 +693,17 @@ __global__ void weighted_values_partial_kernel(const float* __restrict__ w, cons
         for (int ww = 0; ww < warps; ++ww) s += s_acc[ww][e];
         partial[(size_t)blockIdx.x * D + e] = s;
     }
-}
-
-template <int EPL>
-__global__ void __launch_bounds__(256)
-weighted_values_final_kernel(const float* __restrict__ partial, int nparts, float* __restrict__ out, uint64_t seed,
-                             float inv_sqrt_d) {
-    constexpr int D = 32 * EPL;
-    __shared__ float s_part[8][D];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float v[EPL];
-#pragma unroll
-    for (int k = 0; k < EPL; ++k) v[k] = 0.0f;
-    for (int p = warp; p < nparts; p += 8) {
-#pragma unroll
-        for (int k = 0; k < EPL; ++k) v[k] += partial[(size_t)p * D + lane + 32 * k];
-    }
-#pragma unroll
-    for (int k = 0; k < EPL; ++k) s_part[warp][lane + 32 * k] = v[k];
+    if (ticket == nullptr) return;
+    // the CTA that arrives last adds the partials up: no second launch
+    __shared__ int s_last;
+    __threadfence();
     __syncthreads();
-    if (warp != 0) return;
-#pragma unroll
-    for (int k = 0; k < EPL; ++k) {
-        float s = 0.0f;
-#pragma unroll
-        for (int ww = 0; ww < 8; ++ww) s += s_part[ww][lane + 32 * k];
-        v[k] = s;
-    }
-    wht_lanes<EPL>(v, lane);
-#pragma unroll
-    for (int k = 0; k < EPL; ++k) out[lane + 32 * k] = (v[k] * inv_sqrt_d) * sign_of(seed, lane + 32 * k);
+    if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1 : 0;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    weighted_values_final<EPL>(partial, (int)gridDim.x, out, seed, inv_sqrt_d, s_acc);
+    if (threadIdx.x == 0) *ticket = 0u;   // ready for the next call
 }
 
 // ---- long key / value lists: one lane per 32 consecutive elements ---------------------------------------
@@ -1206,13 +1271,41 @@ int tqb_weighted_values(const tqb_config* cfg, const float* w, const uint8_t* pa
         return check_launch(s);
     }
     TQB_DISPATCH_EPL(cfg->dim, {
-        weighted_values_partial_kernel<EPL><<<nparts, 256, 0, s>>>(w, packed, scales, n, partial, cb, polar.bits, pb);
+        weighted_values_partial_kernel<EPL><<<nparts, 256, 0, s>>>(w, packed, scales, n, partial, cb, polar.bits, pb, nullptr, nullptr, 0, 0.0f);
         weighted_values_final_kernel<EPL><<<1, 256, 0, s>>>(partial, nparts, out, cfg->rotation_seed, host_inv_sqrt(cfg->dim));
     });
     return check_launch(s);
 }
 
 }  // extern "C"
+
+// The two calls of QuantizedKVCache on short lists, one launch each.  `scores` / `w` / `out` may be mapped host memory.
+// TQB_ERR_UNSUPPORTED: the list is long, take the table kernels.
+int tqb::launch_scores_query(const tqb_config* cfg, const uint32_t* rbits, const float* q_host, const uint8_t* packed,
+                             const uint16_t* scales, const uint8_t* signs, const uint16_t* rnorms, long long n, float* scores,
+                             cudaStream_t s) {
+    const int dim = cfg->dim, bits = cfg->bits - 1;
+    Codebook cb;
+    if (n >= kListMin || dim > 256 || !whole_codebook(bits, dim, cb)) return TQB_ERR_UNSUPPORTED;
+    QueryArg q{};
+    for (int i = 0; i < dim; ++i) q.q[i] = q_host[i];
+    TQB_DISPATCH_EPL(dim, (scores_query_kernel<EPL><<<grid_warps(n, 8), 256, 0, s>>>(
+        q, rbits, packed, scales, signs, rnorms, n, scores, cb, bits, (int)tqb_packed_bytes(bits, dim), cfg->rotation_seed,
+        host_inv_sqrt(dim), sqrtf((float)dim))));
+    return check_launch(s);
+}
+
+int tqb::launch_weighted_values_one(const tqb_config* cfg, const float* w, const uint8_t* packed, const uint16_t* scales, long long n,
+                                    float* out, float* partial, unsigned* ticket, cudaStream_t s) {
+    const int dim = cfg->dim, bits = cfg->bits - 1;
+    Codebook cb;
+    if (n >= kListMin || dim > 256 || !whole_codebook(bits, dim, cb)) return TQB_ERR_UNSUPPORTED;
+    int nparts = (int)((n + 7) / 8);
+    if (nparts > kWvBlocks) nparts = kWvBlocks;
+    TQB_DISPATCH_EPL(dim, (weighted_values_partial_kernel<EPL><<<nparts, 256, 0, s>>>(
+        w, packed, scales, n, partial, cb, bits, (int)tqb_packed_bytes(bits, dim), ticket, out, cfg->rotation_seed, host_inv_sqrt(dim))));
+    return check_launch(s);
+}
 
 extern "C" {
 
