@@ -52,53 +52,89 @@ struct DevBuf {
 };
 
 // Blocks of device memory that a cache object gives up (reset, growth) and takes again: cudaMalloc and cudaFree cost
-// about 80 us each and cudaFree waits for the whole device, so a request of 16 steps on 28 layers spent 18 of its 20 ms
-// in them.  The pool belongs to one cache object, keeps at most kKeepBytes and is given back with the object or when
-// an allocation fails.  Every block in it is idle: its owner has synchronised the device before it was put here.
-struct BlockPool {
-    static constexpr size_t kKeepBytes = 512u << 20;
+// 80 to 500 us each and cudaFree waits for the whole device, so a request of 16 steps on 28 layers spent 18 of its 20 ms
+// in them.  Small blocks come from slabs: the layers of a cache grow to the same size one after the other, so the first one
+// asks for all that are as far behind (a new cache's 28 layers of 1,024 tokens stored: 9.1 -> 0.9 ms).
+// The pool belongs to one cache object, keeps at most kKeepBytes idle and is given back with the object or when an allocation
+// fails.  Every idle block is unused: its owner has synchronised the device before it was put here.
+class BlockPool {
+public:
+    static constexpr size_t kKeepBytes = 512u << 20, kSlabBytes = 64u << 20;
     struct Block {
-        void* p;
-        size_t bytes;
+        void* p = nullptr;
+        size_t bytes = 0;
+        int slab = -1;
     };
-    std::vector<Block> idle;
-    size_t held = 0;
 
-    // The smallest idle block that fits, unless it is more than twice as large; else a new one.  `use_idle` = false while
-    // the stream is being captured: whatever cudaMalloc answers there is the answer.
-    cudaError_t take(size_t need, bool use_idle, void** p, size_t* bytes) {
-        size_t best = idle.size();
-        for (size_t i = 0; use_idle && i < idle.size(); ++i)
-            if (idle[i].bytes >= need && idle[i].bytes / 2 <= need && (best == idle.size() || idle[i].bytes < idle[best].bytes)) best = i;
-        if (best != idle.size()) {
-            *p = idle[best].p;
-            *bytes = idle[best].bytes;
-            held -= idle[best].bytes;
-            idle.erase(idle.begin() + best);
-            return cudaSuccess;
-        }
-        cudaError_t e = cudaMalloc(p, need);
-        if (e == cudaErrorMemoryAllocation && !idle.empty()) {
+    // The smallest idle block that fits, unless it is more than twice as large; else a new one, out of a slab of up to
+    // `alike` blocks of the size.  `use_idle` = false while the stream is being captured: whatever cudaMalloc answers there is the answer.
+    cudaError_t take(size_t need, int alike, bool use_idle, Block* out) {
+        if (use_idle && take_idle(need, out)) return cudaSuccess;
+        int count = use_idle && need <= kSlabBytes / 2 ? (int)std::min<size_t>((size_t)alike, kSlabBytes / need) : 1;
+        if (count < 1) count = 1;
+        void* p = nullptr;
+        cudaError_t e = cudaMalloc(&p, need * count);
+        if (e == cudaErrorMemoryAllocation && (count > 1 || !idle_.empty())) {
             cudaGetLastError();
             trim();
-            e = cudaMalloc(p, need);
+            count = 1;
+            e = cudaMalloc(&p, need);
         }
-        *bytes = need;
-        return e;
+        if (e != cudaSuccess) return e;
+        const int slab = (int)slabs_.size();
+        slabs_.push_back(Slab{p, count, count});
+        for (int i = 1; i < count; ++i) put(Block{(char*)p + i * need, need, slab});
+        *out = Block{p, need, slab};
+        return cudaSuccess;
     }
-    void put(void* p, size_t bytes) {
-        if (!p) return;
-        if (held + bytes > kKeepBytes) {
-            cudaFree(p);
-            return;
-        }
-        idle.push_back(Block{p, bytes});
-        held += bytes;
+    void put(const Block& b) {
+        if (!b.p) return;
+        idle_.push_back(b);
+        held_ += b.bytes;
+        --slabs_[b.slab].used;
+        if (held_ > kKeepBytes) trim();
     }
+    // Frees what no live block shares a slab with.
     void trim() {
-        for (auto& b : idle) cudaFree(b.p);
-        idle.clear();
-        held = 0;
+        for (size_t i = 0; i < slabs_.size(); ++i)
+            if (slabs_[i].used == 0 && slabs_[i].p) {
+                for (size_t k = idle_.size(); k-- > 0;)
+                    if (idle_[k].slab == (int)i) {
+                        held_ -= idle_[k].bytes;
+                        idle_.erase(idle_.begin() + k);
+                    }
+                cudaFree(slabs_[i].p);
+                slabs_[i].p = nullptr;
+            }
+    }
+    // With the object: live blocks too.
+    void release() {
+        for (auto& s : slabs_)
+            if (s.p) cudaFree(s.p);
+        slabs_.clear();
+        idle_.clear();
+        held_ = 0;
+    }
+
+private:
+    struct Slab {
+        void* p;
+        int blocks, used;
+    };
+    std::vector<Block> idle_;
+    std::vector<Slab> slabs_;
+    size_t held_ = 0;
+
+    bool take_idle(size_t need, Block* out) {
+        size_t best = idle_.size();
+        for (size_t i = 0; i < idle_.size(); ++i)
+            if (idle_[i].bytes >= need && idle_[i].bytes / 2 <= need && (best == idle_.size() || idle_[i].bytes < idle_[best].bytes)) best = i;
+        if (best == idle_.size()) return false;
+        *out = idle_[best];
+        held_ -= out->bytes;
+        ++slabs_[out->slab].used;
+        idle_.erase(idle_.begin() + best);
+        return true;
     }
 };
 
@@ -145,8 +181,7 @@ struct tqb_pqo_cache {
         uint16_t *ks = nullptr, *vs = nullptr;
         int64_t cap = 0, len = 0;
         bool active = false;
-        void* block = nullptr;   // one allocation: K indices, V indices, K scales, V scales, each 256-byte aligned
-        size_t block_bytes = 0;
+        BlockPool::Block block;   // K indices, V indices, K scales, V scales, each 256-byte aligned
     };
     std::vector<Layer> layers;
     BlockPool pool;
@@ -195,7 +230,7 @@ struct tqb_pqo_cache {
 
     // (nothing queued uses the layer any more)
     void free_layer(Layer& l) {
-        pool.put(l.block, l.block_bytes);
+        pool.put(l.block);
         l = Layer{};
     }
 
@@ -214,15 +249,17 @@ struct tqb_pqo_cache {
         const size_t sb = (size_t)heads * new_cap * nblk * sizeof(uint16_t);
         const size_t ia = align256(ib), sa = align256(sb);
         cudaError_t e;
-        if ((e = pool.take(2 * (ia + sa), !capturing(s), &nl.block, &nl.block_bytes)) != cudaSuccess) return cuda_fail(e);
-        nl.ki = (uint8_t*)nl.block;
+        int alike = 0;   // layers that will ask for the same next
+        for (const auto& o : layers) alike += o.cap < needed ? 1 : 0;
+        if ((e = pool.take(2 * (ia + sa), alike, !capturing(s), &nl.block)) != cudaSuccess) return cuda_fail(e);
+        nl.ki = (uint8_t*)nl.block.p;
         nl.vi = nl.ki + ia;
         nl.ks = (uint16_t*)(nl.vi + ia);
         nl.vs = (uint16_t*)(nl.vi + ia + sa);
         // on any failure from here on the new buffers are released and the layer is left as it was
         auto fill = [&]() -> cudaError_t {
             cudaError_t r;
-            if ((r = cudaMemsetAsync(nl.block, 0, 2 * (ia + sa), s)) != cudaSuccess) return r;
+            if ((r = cudaMemsetAsync(nl.block.p, 0, 2 * (ia + sa), s)) != cudaSuccess) return r;
             if (l.len > 0) {
                 const size_t iw = (size_t)l.len * packed_dim, sw = (size_t)l.len * nblk * 2;
                 if ((r = cudaMemcpy2DAsync(nl.ki, (size_t)new_cap * packed_dim, l.ki, (size_t)l.cap * packed_dim, iw, heads,
@@ -239,7 +276,7 @@ struct tqb_pqo_cache {
         };
         if ((e = fill()) != cudaSuccess) {
             cudaDeviceSynchronize();   // nothing queued may still write the buffers that are released next
-            cudaFree(nl.block);
+            free_layer(nl);
             return cuda_fail(e);
         }
         if (l.ki) free_layer(l);
@@ -424,8 +461,7 @@ int tqb_pqo_cache_create(const tqb_cache_config* cfg, tqb_pqo_cache** out) {
 
 void tqb_pqo_cache_destroy(tqb_pqo_cache* c) {
     if (!c) return;
-    for (auto& l : c->layers) cudaFree(l.block);   // waits for the device
-    c->pool.trim();
+    c->pool.release();   // waits for the device
     c->stage_k.release(); c->stage_v.release(); c->stage_q.release(); c->stage_out.release(); c->scratch.release();
     c->destroy_pipeline();
     delete c;
@@ -1023,7 +1059,7 @@ struct tqb_tq_cache {
         uint8_t* signs = nullptr;
         uint16_t* norms = nullptr;
         int64_t cap = 0;
-        size_t block_bytes = 0;   // one allocation that starts at `signs`
+        BlockPool::Block block;   // signs, then norms
     };
     std::vector<Q> qjl;
     uint32_t* rbits = nullptr;
@@ -1032,7 +1068,7 @@ struct tqb_tq_cache {
     int sb() const { return base->cfg.head_dim / 8; }
 
     void free_q(Q& q) {
-        base->pool.put(q.signs, q.block_bytes);
+        base->pool.put(q.block);
         q = Q{};
     }
 
@@ -1046,7 +1082,10 @@ struct tqb_tq_cache {
         const int heads = base->heads;
         const size_t sa = align256((size_t)heads * new_cap * sb()), bytes = sa + align256((size_t)heads * new_cap * 2);
         cudaError_t e;
-        if ((e = base->pool.take(bytes, !capturing(s), (void**)&n.signs, &n.block_bytes)) != cudaSuccess) return cuda_fail(e);
+        int alike = 0;
+        for (const auto& o : qjl) alike += o.cap < needed ? 1 : 0;
+        if ((e = base->pool.take(bytes, alike, !capturing(s), &n.block)) != cudaSuccess) return cuda_fail(e);
+        n.signs = (uint8_t*)n.block.p;
         n.norms = (uint16_t*)(n.signs + sa);
         auto fill = [&]() -> cudaError_t {
             cudaError_t r;
@@ -1061,7 +1100,7 @@ struct tqb_tq_cache {
         };
         if ((e = fill()) != cudaSuccess) {
             cudaDeviceSynchronize();
-            cudaFree(n.signs);
+            free_q(n);
             return cuda_fail(e);
         }
         if (q.signs) free_q(q);
@@ -1159,7 +1198,6 @@ int tqb_tq_cache_create(const tqb_cache_config* cfg, tqb_tq_cache** out) {
 
 void tqb_tq_cache_destroy(tqb_tq_cache* c) {
     if (!c) return;
-    for (auto& q : c->qjl) cudaFree(q.signs);
     if (c->rbits) cudaFree(c->rbits);
     c->deq.release(); c->qf32.release(); c->rq.release();
     tqb_pqo_cache_destroy(c->base);
