@@ -19,15 +19,15 @@
 // the even and the odd tiles, merged once at the end like two split-K partitions.  Thread r of a group owns query
 // row r = tensor-memory lane r, so the online softmax needs no shuffles; the output is rotated back in registers
 // (one 32-point butterfly per block) at the end.
-// Measured (B200, 32 q / 8 KV heads, 4-bit, bf16): 512 queries on 7,680 tokens 98 us = 670 TFLOP/s of causal attention math.
+// Measured (B200, 32 q / 8 KV heads, 4-bit, bf16): 512 queries on 7,680 tokens 96 us = 690 TFLOP/s of causal attention math.
 // It took 134 us with the queries rotated a warp per block (34 dependent loads before the first tile), one f32
 // operation an instruction in the softmax, and the CTAs started in ascending order of their work; a 1,999-token prompt's
 // call (store + attend) went from 120 - 150 to 67 us, of which two transposing passes over q and out were 23.
 // The f16 roundings of Q~, K~, P and V are this kernel's error budget (a few 1e-4 of the value range on the outputs;
 // the decode kernels, which keep the query in f32 or as 20-bit integers, stay below 1e-5).
 //
-// Warp roles: warps 0-3 / 4-7 softmax group 0 / 1 (correction, epilogue), warps 8-9 load and unpack K tiles, warps
-// 10-13 V tiles (two stages each), warp 14 issues the MMAs.  All hand-offs go through mbarriers; every wait is
+// Warp roles: warps 0-3 / 4-7 softmax group 0 / 1 (correction, epilogue), warps 8-11 load and unpack K tiles, warps
+// 12-15 V tiles (two stages each), warp 16 issues the MMAs: every SM sub-core has two softmax, one K and one V warp.  All hand-offs go through mbarriers; every wait is
 // bounded and a wait that runs out sets a flag, drains and returns (tqb_chunk_umma_timeouts).
 #include <cuda.h>
 #include <float.h>
@@ -44,7 +44,7 @@ namespace {
 constexpr int kRows = 128;          // query rows per CTA
 constexpr int kTile = 64;           // cache tokens per step
 constexpr int kD = 128;
-constexpr int kThreads = 15 * 32;
+constexpr int kThreads = 17 * 32;
 constexpr float kNegBig = -1.0e30f;
 
 // shared-memory map (bytes from a 1024-aligned base)
@@ -208,7 +208,8 @@ __device__ __forceinline__ int perm4(int p) { return (p >> 1) + 4 * (p & 1); }
 // 16 consecutive bytes of a swizzled 128-byte row: chunk c of row `row` of a tile whose rows are 128 bytes apart
 __device__ __forceinline__ uint32_t sw128(int row, int chunk) { return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4)); }
 
-// ---- load + unpack role: IS_K ? warps 8-9 (K tiles, four pieces per thread) : warps 10-13 (V tiles, two pieces) ----
+// ---- load + unpack role: warps 8-11 (K tiles), 12-15 (V tiles); two pieces per thread and tile ----
+// (two warps for K, four pieces a thread: 97.6 against 95.6 us at 512 queries on 7,680 tokens)
 // A piece is one (token, block): 32 codes and their scale.  Eight consecutive lanes take the eight tokens of one token
 // group (eight distinct swizzle phases, so the 16-byte stores of a quarter-warp fall into eight different bank
 // groups), the four lane octets take the four blocks.  The packed pieces are fetched two tiles ahead of their use
@@ -218,7 +219,7 @@ __device__ __forceinline__ uint32_t sw128(int row, int chunk) { return (uint32_t
 template <int BITS, bool IS_K>
 __device__ __forceinline__ bool unpack_role(const ChunkArgs& a, unsigned char* sm, uint32_t bar_full, uint32_t bar_empty, int w2, int lane,
                                             size_t row0, int kv_hi, int ntiles) {
-    constexpr int NP = IS_K ? 4 : 2;             // pieces per thread and tile
+    constexpr int NP = 2;                        // pieces per thread and tile
     constexpr int TSTEP = kTile / NP;            // token distance between a thread's pieces
     const int tl = 8 * w2 + (lane & 7), b = lane >> 3;
     const uint8_t* src_b = IS_K ? a.kb : a.vb;
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
         s_fail = 0;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            mbar_init(bar + kKFull + 8 * i, 128);    // 64 threads, two tiles per stage
+            mbar_init(bar + kKFull + 8 * i, 256);    // 128 threads, two tiles per stage
             mbar_init(bar + kKEmpty + 8 * i, 1);
             mbar_init(bar + kSFull + 8 * i, 1);
             mbar_init(bar + kVFull + 8 * i, 128);
@@ -382,11 +383,11 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
     const uint32_t tmem = s_tmem;
     const uint32_t tmemS = tmem, tmemO = tmem + 256;   // S buffer b at columns 128 b; O of softmax group G at 256 + 128 G
 
-    if (warp >= 8 && warp < 10) {
+    if (warp >= 8 && warp < 12) {
         if (!unpack_role<BITS, true>(a, sm, bar + kKFull, bar + kKEmpty, warp - 8, lane, row0, kv_hi, ntiles)) atomicExch(&s_fail, 1);
-    } else if (warp >= 10 && warp < 14) {
-        if (!unpack_role<BITS, false>(a, sm, bar + kVFull, bar + kVEmpty, warp - 10, lane, row0, kv_hi, ntiles)) atomicExch(&s_fail, 1);
-    } else if (warp == 14) {
+    } else if (warp >= 12 && warp < 16) {
+        if (!unpack_role<BITS, false>(a, sm, bar + kVFull, bar + kVEmpty, warp - 12, lane, row0, kv_hi, ntiles)) atomicExch(&s_fail, 1);
+    } else if (warp == 16) {
         // ================= MMA issue (one lane) =================
         if (lane == 0) {
             constexpr uint32_t idescS = umma_idesc(2 * kTile, false), idescO = umma_idesc(kD, true);
