@@ -295,7 +295,7 @@ residual_sketch_mma_kernel(const T* __restrict__ x, const float* __restrict__ xh
 // precompute_query_projections (src/qjl.rs:488-492) of many queries: a lane owns sign rows lane, lane + 32, ... and adds,
 // left to right, for eight queries at a time, so a +-1 made from a bit (two instructions) serves eight additions
 // (fma(q, +-1, s) rounds once, like s +- q).  One query per warp spends three instructions on every addition:
-// 65,536 queries of 128 dims 117 -> 77 us, 4,096 queries 13.1 -> 12.3 us.
+// 65,536 queries of 128 dims 117 -> 65 us (77 us with one query an instruction), 4,096 queries 13.1 -> 12.3 us.
 constexpr int kProjQ = 8, kProjWarps = 4;
 template <int W, typename T>
 __global__ void __launch_bounds__(kProjWarps * 32)
@@ -317,11 +317,11 @@ projections_tile_kernel(const T* __restrict__ q, long long nq, const uint32_t* _
 #pragma unroll 8
         for (int k = 0; k < D / 4; ++k) vec[32 * k + 8 * (lane >> 3) + (lane & 7)] = to_f32<T>(src[4 * k]);
         __syncwarp();
-        float s[W][kProjQ];
+        F2 s[W][kProjQ / 2];   // two queries an instruction
 #pragma unroll
         for (int k = 0; k < W; ++k)
 #pragma unroll
-            for (int i = 0; i < kProjQ; ++i) s[k][i] = 0.0f;
+            for (int i = 0; i < kProjQ / 2; ++i) s[k][i] = f2(0.0f);
 #pragma unroll 1
         for (int cw = 0; cw < W; ++cw) {
             uint32_t rb[W];
@@ -333,12 +333,12 @@ projections_tile_kernel(const T* __restrict__ q, long long nq, const uint32_t* _
                 const float4 hi = *reinterpret_cast<const float4*>(vec + (cw * 32 + c) * kProjQ + 4);
 #pragma unroll
                 for (int k = 0; k < W; ++k) {
-                    const float m = __uint_as_float((rb[k] << 31) | 0x3F800000u);
+                    const F2 m = f2(__uint_as_float((rb[k] << 31) | 0x3F800000u));
                     rb[k] >>= 1;
-                    s[k][0] = fmaf(lo.x, m, s[k][0]); s[k][1] = fmaf(lo.y, m, s[k][1]);
-                    s[k][2] = fmaf(lo.z, m, s[k][2]); s[k][3] = fmaf(lo.w, m, s[k][3]);
-                    s[k][4] = fmaf(hi.x, m, s[k][4]); s[k][5] = fmaf(hi.y, m, s[k][5]);
-                    s[k][6] = fmaf(hi.z, m, s[k][6]); s[k][7] = fmaf(hi.w, m, s[k][7]);
+                    s[k][0] = fma2(f2(lo.x, lo.y), m, s[k][0]);
+                    s[k][1] = fma2(f2(lo.z, lo.w), m, s[k][1]);
+                    s[k][2] = fma2(f2(hi.x, hi.y), m, s[k][2]);
+                    s[k][3] = fma2(f2(hi.z, hi.w), m, s[k][3]);
                 }
             }
         }
@@ -346,7 +346,10 @@ projections_tile_kernel(const T* __restrict__ q, long long nq, const uint32_t* _
         for (int i = 0; i < kProjQ; ++i)
             if (i < nv)
 #pragma unroll
-                for (int k = 0; k < W; ++k) rq[(q0 + i) * D + lane + 32 * k] = s[k][i] * inv_sqrt_d;
+                for (int k = 0; k < W; ++k) {
+                    const float2 t = halves(s[k][i >> 1]);
+                    rq[(q0 + i) * D + lane + 32 * k] = ((i & 1) ? t.y : t.x) * inv_sqrt_d;
+                }
         __syncwarp();
     }
 }
