@@ -6,6 +6,8 @@
 #include "tqb_common.cuh"
 #include "tqb_f32x2.cuh"
 
+#include <type_traits>
+
 namespace tqb {
 
 template <typename T>
@@ -42,6 +44,29 @@ __device__ __forceinline__ void load32<__half>(const __half* p, float (&v)[32]) 
             float2 f = __half22float2(h[i]);
             v[8 * k + 2 * i] = f.x;
             v[8 * k + 2 * i + 1] = f.y;
+        }
+    }
+}
+
+// 32 values from 16-byte pieces in shared memory
+template <typename T>
+__device__ __forceinline__ void unpack32(const unsigned char* p, float (&v)[32]) {
+    constexpr int kPer = 16 / (int)sizeof(T);
+#pragma unroll
+    for (int k = 0; k < 32 / kPer; ++k) {
+        const uint4 r = *reinterpret_cast<const uint4*>(p + 16 * k);
+        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if constexpr (sizeof(T) == 4) v[4 * k + i] = __uint_as_float(w[i]);
+            else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+                v[8 * k + 2 * i] = __uint_as_float(w[i] << 16);
+                v[8 * k + 2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+            } else {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                v[8 * k + 2 * i] = f.x;
+                v[8 * k + 2 * i + 1] = f.y;
+            }
         }
     }
 }
@@ -89,26 +114,22 @@ __device__ __forceinline__ void build_cell_table(const Codebook& cb, int n_bnd, 
     }
 }
 
-// x: the block's 32 input values (16-byte aligned).  w: packed codes (4 * BITS bytes, LSB-first), returns the
+// v (x, 16-byte aligned): the block's 32 input values.  w: packed codes (4 * BITS bytes, LSB-first), returns the
 // f32 scale (before the outlier sign).  cb: the codebook.  lut: the caller's lane of the cell table in
 // shared memory (build_cell_table, + lane), or nullptr for the register bisection.  TABLE: the codebook is not the
 // 4-bit uniform grid even when BITS = 4 (codes of a narrower codebook stored at BITS width); needs lut.
 // Two values per instruction throughout (elements i and i + 16); the codes are whole f32 numbers that are packed by
 // multiply-adds (16 or 24 bits of them are exact) instead of a mask, a shift and an add each.
-template <typename T, int BITS, bool TABLE = false>
-__device__ __forceinline__ float pqo_quantize_block(const T* x, const Codebook& cb, float outer_centroid, uint32_t (&w)[4],
-                                                    const float2* lut = nullptr) {
+template <int BITS, bool TABLE = false>
+__device__ __forceinline__ float pqo_quantize_values(const float (&v)[32], const Codebook& cb, float outer_centroid, uint32_t (&w)[4],
+                                                     const float2* lut = nullptr) {
     const float inv_sqrt = 1.0f / sqrtf((float)kBlock);
     const float R = cb.c[(1 << BITS) - 1];
     const float inv_step = 15.0f / (2.0f * R);
     const float kMagic = 12582912.0f;          // 1.5 * 2^23
     F2 p[16];
-    {
-        float v[32];
-        load32<T>(x, v);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) p[i] = f2(v[i], v[i + 16]);
-    }
+    for (int i = 0; i < 16; ++i) p[i] = f2(v[i], v[i + 16]);
     butterfly32_pairs(p);
     float amax_w = 0.0f;
 #pragma unroll
@@ -139,9 +160,9 @@ __device__ __forceinline__ float pqo_quantize_block(const T* x, const Codebook& 
         if (far > 0.49998f) {   // rare: exact division and the f32 boundary table
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-                const float2 v = halves(p[i]);
-                const float t0 = __fdiv_rn((v.x * inv_sqrt) * (((kSignMask >> i) & 1u) ? -1.0f : 1.0f), scale);
-                const float t1 = __fdiv_rn((v.y * inv_sqrt) * (((kSignMask >> (i + 16)) & 1u) ? -1.0f : 1.0f), scale);
+                const float2 v2 = halves(p[i]);
+                const float t0 = __fdiv_rn((v2.x * inv_sqrt) * (((kSignMask >> i) & 1u) ? -1.0f : 1.0f), scale);
+                const float t1 = __fdiv_rn((v2.y * inv_sqrt) * (((kSignMask >> (i + 16)) & 1u) ? -1.0f : 1.0f), scale);
                 float c0 = 0.0f, c1 = 0.0f;
 #pragma unroll
                 for (int k = 0; k < 15; ++k) {
@@ -212,6 +233,14 @@ __device__ __forceinline__ float pqo_quantize_block(const T* x, const Codebook& 
         w[3] = 0u;
     }
     return scale;
+}
+
+template <typename T, int BITS, bool TABLE = false>
+__device__ __forceinline__ float pqo_quantize_block(const T* x, const Codebook& cb, float outer_centroid, uint32_t (&w)[4],
+                                                    const float2* lut = nullptr) {
+    float v[32];
+    load32<T>(x, v);
+    return pqo_quantize_values<BITS, TABLE>(v, cb, outer_centroid, w, lut);
 }
 
 }  // namespace tqb
