@@ -410,11 +410,11 @@ int32_t tqb_decode_num_partitions(int32_t num_kv_heads, int32_t kv_len) {
     // faster split in 2 than in 4, and 7 % faster than unsplit (which leaves 14 % of the slots empty); more,
     // shorter partitions pay the per-CTA query prologue and merge again.  So: two residencies' worth of CTAs
     // while a partition keeps at least 768 tokens, else one residency's worth, never below 128 tokens, the step of a
-    // CTA (8 heads x 1,024 tokens: 8 partitions 6.0 us, 16 partitions 7.1 us).  One
+    // CTA (8 heads x 1,024 tokens: 8 partitions 6.0 us, 16 partitions 7.1 us; up to 128 tokens make two of 64).  One
     // residency's worth is rounded DOWN: 64 heads x 10 partitions are 640 CTAs for 592 slots, and the 48 left over
     // start when the first ones end - the launch takes twice as long as with 9 partitions.
     const long long resident = 148 * 4;
-    const int max_p = (kv_len + 127) / 128;
+    const int max_p = kv_len <= 128 ? (kv_len + 63) / 64 : (kv_len + 127) / 128;
     const long long p1 = resident / num_kv_heads;
     long long p2 = 2 * resident / num_kv_heads;
     if (p2 < 1) p2 = 1;
