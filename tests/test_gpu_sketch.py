@@ -118,3 +118,18 @@ def test_decode_input_in_one_launch_equals_separate_kernels(bits, dim, batch, gr
         outs.append(got + [r.k, r.v, r.logit_bias])
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,ulp", [(torch.float32, 2.0 ** -22), (torch.float16, 2.0 ** -10), (torch.bfloat16, 2.0 ** -7)])
+@pytest.mark.parametrize("dim,q_len,batch", [(32, 70, 2), (64, 65, 2), (128, 64, 2), (256, 45, 3)])
+def test_bias_of_many_queries_equals_few(dim, q_len, batch, dtype, ulp):
+    # from 2,048 queries on (2 x 16 x 64) 16-bit ones are projected on the tensor cores; pieces take the sequential sums.  Both
+    # sums are exact to f32 rounding, so the bias differs by its own last place at most
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    cfg = tq.CacheConfig(bits=3, head_dim=dim, num_kv_heads=4, num_layers=1, batch=batch, outlier_blocks=0)
+    k, v = (torch.randn((batch, 4, 50, dim), generator=g, device="cuda").to(dtype) for _ in range(2))
+    q = torch.randn((batch, 16, q_len, dim), generator=g, device="cuda").to(dtype)
+    many = tq.TqCache(cfg).prefill(0, k, v, q).logit_bias
+    few = torch.cat([tq.TqCache(cfg).prefill(0, k, v, q[:, :, a:a + 33].contiguous()).logit_bias for a in range(0, q_len, 33)], dim=2)
+    scale = few.float().abs().max()
+    assert ((many.float() - few.float()).abs() <= ulp * few.float().abs() + 2.0 ** -20 * scale).all()

@@ -443,6 +443,89 @@ int launch_append(const TqAppend& a, const Codebook& cb, float outer, float sign
     return check_launch(s);
 }
 
+// The same for 16-bit queries on the tensor cores, 16 to a warp: a bf16 value is one bf16 term and an f16 value two, so every
+// product with +-1 is exact and only the f32 accumulation rounds - over fewer steps than the sum element by element.
+// Measured (24,576 queries of 128 dims, bf16): 27 -> 14 us; relative error against 64 bits 2.58e-8 (element by element 2.59e-8),
+// at a log-normal spread of 2 over the elements 6.8e-8 (9.3e-8).
+template <int W, typename T>
+__global__ void __launch_bounds__(kSketchWarps<W> * 32)
+projections_mma_kernel(const T* __restrict__ q, long long nq, const uint32_t* __restrict__ rbits, float* __restrict__ rq, float inv_sqrt_d) {
+    static_assert(sizeof(T) == 2, "f32 queries: projections_tile_kernel");
+    constexpr int D = 32 * W, P = D + 4, NW = kSketchWarps<W>, NT = W < 4 ? 4 * W : 16;
+    constexpr int kTerms = std::is_same<T, __nv_bfloat16>::value ? 1 : 2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint32_t* s_rb = reinterpret_cast<uint32_t*>(smem_raw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = lane >> 2, j = lane & 3;
+    float* tile = reinterpret_cast<float*>(s_rb + D * (W + 1)) + warp * kTileVec * P;
+    load_rbits<W>(s_rb, rbits);
+    __syncthreads();
+    const long long tiles = (nq + kTileVec - 1) / kTileVec;
+    for (long long t0 = (long long)blockIdx.x * NW + warp; t0 < tiles; t0 += (long long)gridDim.x * NW) {
+        const long long q0 = t0 * kTileVec;
+        const int nv = (int)min((long long)kTileVec, nq - q0);
+#pragma unroll 4
+        for (int i = lane; i < kTileVec * D / 4; i += 32) {
+            const int r = i / (D / 4), c = i % (D / 4);
+            T e[4];
+            *reinterpret_cast<uint2*>(e) = __ldg(reinterpret_cast<const uint2*>(q + (q0 + min(r, nv - 1)) * D + 4 * c));
+            *reinterpret_cast<float4*>(tile + r * P + 4 * c) = make_float4(to_f32<T>(e[0]), to_f32<T>(e[1]), to_f32<T>(e[2]), to_f32<T>(e[3]));
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int pass = 0; pass < 4 * W / NT; ++pass) {
+            float acc[NT][4];
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[t][e] = 0.0f;
+#pragma unroll 1
+            for (int w = 0; w < W; ++w) {
+                uint32_t a[2][2][4];   // [half][term][fragment register], k-slots as in sketch_tile
+                const float* e0 = tile + n * P + 32 * w + j;
+                const float* e1 = e0 + 8 * P;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    split2(e0[8 * h], e0[8 * h + 16], a[h][0][0], a[h][1][0]);
+                    split2(e1[8 * h], e1[8 * h + 16], a[h][0][1], a[h][1][1]);
+                    split2(e0[8 * h + 4], e0[8 * h + 20], a[h][0][2], a[h][1][2]);
+                    split2(e1[8 * h + 4], e1[8 * h + 20], a[h][0][3], a[h][1][3]);
+                    if (kTerms == 2) {   // an infinity leaves no second term (Inf - Inf)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if ((a[h][0][e] & 0x7F80u) == 0x7F80u) a[h][1][e] &= 0xFFFF0000u;
+                            if ((a[h][0][e] & 0x7F800000u) == 0x7F800000u) a[h][1][e] &= 0x0000FFFFu;
+                        }
+                    }
+                }
+                const uint32_t* rb = s_rb + (pass * NT * 8 + n) * (W + 1) + w;
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    const uint32_t u = rb[t * 8 * (W + 1)] << (3 - j);
+                    uint32_t b[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) b[c] = ((u << (12 - 4 * c)) & 0x80008000u) | 0x3F803F80u;
+                    // 32 dims at a time: the tensor cores' own accumulation truncates, the additions of the parts round
+                    float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int term = kTerms - 1; term >= 0; --term) {   // the small terms first
+                        mma_bf16(part, a[0][term], b[0], b[1]);
+                        mma_bf16(part, a[1][term], b[2], b[3]);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[t][e] += part[e];
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                float* o = rq + (q0 + n) * D + (pass * NT + t) * 8 + 2 * j;
+                if (n < nv) *reinterpret_cast<float2*>(o) = make_float2(acc[t][0] * inv_sqrt_d, acc[t][1] * inv_sqrt_d);
+                if (n + 8 < nv) *reinterpret_cast<float2*>(o + 8 * D) = make_float2(acc[t][2] * inv_sqrt_d, acc[t][3] * inv_sqrt_d);
+            }
+        }
+        __syncwarp();
+    }
+}
+
 template <typename K>
 int opt_in(K kernel, size_t smem) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -478,6 +561,18 @@ int launch_residual(const T* x, const float* xhat, long long n, const uint32_t* 
 
 template <int W, typename T>
 int launch_projections(const T* q, long long nq, const uint32_t* rbits, float* rq, float inv, cudaStream_t s) {
+    if constexpr (sizeof(T) == 2) {
+        if (((uintptr_t)q % 8) == 0 && ((uintptr_t)rq % 8) == 0) {
+            constexpr int NW = kSketchWarps<W>;
+            const size_t smem = sketch_smem<W>(0);
+            const int st = opt_in(projections_mma_kernel<W, T>, smem);
+            if (st != TQB_OK) return st;
+            long long tiles = (nq + NW * kTileVec - 1) / (NW * kTileVec);
+            if (tiles > 148 * 2) tiles = 148 * 2;
+            projections_mma_kernel<W, T><<<(int)tiles, NW * 32, smem, s>>>(q, nq, rbits, rq, inv);
+            return check_launch(s);
+        }
+    }
     long long grid = (nq + kProjQ * kProjWarps - 1) / (kProjQ * kProjWarps);
     if (grid > 148 * 8) grid = 148 * 8;
     projections_tile_kernel<W, T><<<(int)grid, kProjWarps * 32, 0, s>>>(q, nq, rbits, rq, inv);

@@ -43,7 +43,7 @@ int launch_residual_sketch(int dim, const void* x, int dtype, const float* xhat,
                            cudaStream_t s);
 
 constexpr long long kProjTileMin = 2048;   // below, one query per warp fills the chip
-// Projections of nq queries of `dtype`, eight to a warp: bit for bit those of projections_kernel.
+// Projections of nq queries of `dtype`: f32 queries bit for bit as projections_kernel gives them, 16-bit ones on the tensor cores.
 int launch_projections_tile(int dim, const void* q, int dtype, long long nq, const uint32_t* rbits, float* rq, float inv_sqrt_d,
                             cudaStream_t s);
 
