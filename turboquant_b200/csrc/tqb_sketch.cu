@@ -561,7 +561,8 @@ int launch_residual(const T* x, const float* xhat, long long n, const uint32_t* 
 
 template <int W, typename T>
 int launch_projections(const T* q, long long nq, const uint32_t* rbits, float* rq, float inv, cudaStream_t s) {
-    if constexpr (sizeof(T) == 2) {
+    // (32 dims are one part: there the sum element by element is the closer one, 4.6e-8 against 5.7e-8 at a wide spread)
+    if constexpr (sizeof(T) == 2 && W > 1) {
         if (((uintptr_t)q % 8) == 0 && ((uintptr_t)rq % 8) == 0) {
             constexpr int NW = kSketchWarps<W>;
             const size_t smem = sketch_smem<W>(0);
