@@ -164,6 +164,41 @@ def test_fused_append_equals_append_then_attend(bits, nm, ob, dtype, L):
             assert (got.float() - want.float()).abs().max() < (1e-2 if dtype == torch.bfloat16 else 1e-5)
 
 
+@pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("g", [4, 8])
+@pytest.mark.parametrize("tma", [False, True])
+# (length, partitions): 0 is the default, two partitions of 64 up to 128 tokens.  The others leave a partition an odd number of
+# 64-token steps and the last partition 1 to 64 tokens: a step of two groups must not reach into the row being appended.
+@pytest.mark.parametrize("L,parts", [(65, 0), (66, 0), (100, 0), (127, 0), (128, 0), (193, 2), (256, 2), (385, 3), (448, 3), (700, 4), (1000, 6)])
+def test_fused_append_ignores_what_the_row_held_before(bits, g, tma, L, parts):
+    rng = np.random.default_rng(bits * 1000 + g * 100 + L)
+    hkv, stride = 8, L + 2
+    ki, ks, vi, vs = (dev(x) for x in make_cache(rng, hkv, L - 1, stride, bits))
+    ks, vs = ks.view(torch.int16), vs.view(torch.int16)
+    newk = torch.from_numpy(rng.standard_normal((hkv, 128)).astype(np.float32)).cuda()
+    newv = torch.from_numpy(rng.standard_normal((hkv, 128)).astype(np.float32)).cuda()
+    q = torch.from_numpy((rng.standard_normal((hkv * g, 128)) / np.sqrt(128)).astype(np.float32)).cuda()
+    for t in (ki, vi):
+        t[:, L - 1:] = 0xFF
+    ref = [t.clone() for t in (ki, ks, vi, vs)]
+    tq.block_quantize(newk, bits, out=(ref[0], ref[1]), rows_per_group=1, group_stride=stride, row_offset=L - 1)
+    tq.block_quantize(newv, bits, out=(ref[2], ref[3]), rows_per_group=1, group_stride=stride, row_offset=L - 1)
+    want = tq.decode_attention(q, *ref, L, bits, 0.0884, num_partitions=parts, tma=tma)
+    assert torch.isfinite(want).all()
+    for scale in (0x7E00, 0x7C00, -0x400):       # f16 NaN, Inf, -Inf in the scales of the row and of what lies behind it
+        got_cache = [torch.empty_like(t) for t in ref]
+        got = []
+        for _ in range(40):
+            for dst, src in zip(got_cache, (ki, ks, vi, vs)):
+                dst.copy_(src)
+            got_cache[1][:, L - 1:] = scale
+            got_cache[3][:, L - 1:] = scale
+            got.append(tq.decode_attention(q, *got_cache, L, bits, 0.0884, num_partitions=parts, tma=tma, append=(newk, newv)))
+        for dst, src in zip(got_cache, ref):
+            assert torch.equal(dst[:, :L], src[:, :L])
+        assert all(torch.equal(x, want) for x in got)
+
+
 @pytest.mark.parametrize("bits,nm,ob", [(3, 0, -1), (3, 1, -1), (3, 0, 0), (4, 0, -1)])
 def test_tensor_core_kernel_sharp_softmax(bits, nm, ob):
     # large logits: a handful of tokens carry all the weight, so element errors are not averaged away.

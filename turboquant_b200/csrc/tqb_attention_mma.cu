@@ -386,8 +386,8 @@ __device__ __forceinline__ FillPlan make_plan(const MmaArgs& a, size_t row0, int
 }
 
 // Issues the copies of the 16 tokens starting at `gs` (where the plan's pointers stand) into the stage at
-// shared address `st`, then moves the pointers on by `stride` tokens.  In the final group of a sequence rows
-// past the last valid token re-read the last token (they are masked later).
+// shared address `st`, then moves the pointers on by `stride` tokens.  Rows past token `last` re-read it (`ragged`; they are
+// masked later).
 template <int BITS>
 __device__ __forceinline__ void stage_fill(FillPlan& f, bool issue, bool ragged, int stride, int gs, int last, uint32_t st) {
     using G = Geo<BITS>;
@@ -502,12 +502,15 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
     const int t_end = min(t_begin + a.part_size, kv_len);
     const size_t row0 = (size_t)cache_head * a.kv_stride;
     const int last = kv_len - 1;
+    // The last token this CTA may read: copies of a group that runs past it re-read it.  Not `last`: another CTA of the
+    // launch may be appending that row, whose old scales may be Inf or NaN and outlive a zero probability.
+    const int own_last = t_end - 1;
     const int first = t_begin + warp * kGroup;
     const int stride = kWarps * kGroup;
     const int ngroups = first < t_end ? (t_end - first + stride - 1) / stride : 0;
     if (a.app_k != nullptr && last >= t_begin && last < t_end) {
-        // Fused append.  Only this CTA ever reads row `last` of this KV head, so a block-wide barrier after
-        // the stores is all the ordering needed.  One thread per 32-block: warp w takes block w of K (lane 0)
+        // Fused append.  Only this CTA ever reads row `last` of this KV head (no copy of a partition goes past its own
+        // end, see `own_last`), so a block-wide barrier after the stores is all the ordering needed.  One thread per 32-block: warp w takes block w of K (lane 0)
         // and of V (lane 1); same code, same bits as block_quantize_pqo_kernel.
         if (lane < 2) {
             const bool is_v = lane == 1;
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
     const uint32_t full0 = (uint32_t)__cvta_generic_to_shared(&s_bar[0][0]);
     const uint32_t empty0 = (uint32_t)__cvta_generic_to_shared(&s_bar[1][0]);
     const int ntiles = t_begin < t_end ? (t_end - t_begin + stride - 1) / stride : 0;   // 64-token tiles of the CTA
-    // (the last step may hold a group past the end: it re-reads the last token and is masked)
+    // (the last step may hold a group past the end: it re-reads the last token - TMA: the last tile - and is masked)
     const int nsteps = ((TMA ? ntiles : ngroups) + kU - 1) / kU * kU;
     const int trow0 = (int)row0 + t_begin;                     // TMA: token row of tile 0 in the whole array
     const bool producer = TMA && tid == 0;
@@ -565,13 +568,13 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 #pragma unroll
             for (int i = 0; i < kAhead; ++i)
-                if (i < nsteps) tma_tile_fill<BITS>(maps, rings_base + i * G::kTileB, full0 + 8 * i, trow0 + i * stride);
+                if (i < nsteps) tma_tile_fill<BITS>(maps, rings_base + i * G::kTileB, full0 + 8 * i, trow0 + min(i, ntiles - 1) * stride);
         }
         // the other threads first touch a barrier after the block-wide barriers of the query prologue
     } else {
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
-            stage_fill<BITS>(plan, i < nsteps, first + i * stride + kGroup > last + 1, stride, first + i * stride, last, ring + i * G::kStageB);
+            stage_fill<BITS>(plan, i < nsteps, first + i * stride + kGroup > t_end, stride, first + i * stride, own_last, ring + i * G::kStageB);
             cp_async_commit();
         }
     }
@@ -774,7 +777,7 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
     auto qjl_fetch = [&](int it, uint32_t (&sg)[2], uint32_t (&nr)[2]) {
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-            const size_t row = row0 + (size_t)min(first + it * stride + n + 8 * t, last);
+            const size_t row = row0 + (size_t)min(first + it * stride + n + 8 * t, own_last);
             sg[t] = __ldg(a.qjl_signs + row * 4 + j);
             nr[t] = __ldg(a.qjl_norms + row);
         }
@@ -798,9 +801,7 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
 #pragma unroll
             for (int i = 0; i < 4; ++i) o[b][m][i] = 0.0f;
 
-    // Loop control in terms of iteration numbers fixed before the loop: the last step that still refills a
-    // stage, the step whose refill is the (only possibly) ragged last group, and the first step with tokens to mask.
-    const int rag_fill = (last + 1 - kGroup - first < 0) ? 0 : (last + 1 - kGroup - first) / stride + 1;   // the first group that runs past the last token
+    // The first group that runs past the partition's end, fixed before the loop: its copies are clamped, its tokens masked.
     const int rag_from = (t_end - kGroup - first < 0) ? 0 : (t_end - kGroup - first) / stride + 1;
     for (int it = 0; it < nsteps; it += kU) {
         uint32_t stu[kU];   // the stages of the step's groups
@@ -812,7 +813,7 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
                 if (producer && it + kAhead + u < nsteps) {
                     // refill the stage of tile it + u - kU once all four warps have released it
                     if (it >= kU && !mbar_wait(empty0 + boff_fill, eparity)) stage_ok = false;
-                    else tma_tile_fill<BITS>(maps, st_fill, full0 + boff_fill, trow0 + (it + kAhead + u) * stride);
+                    else tma_tile_fill<BITS>(maps, st_fill, full0 + boff_fill, trow0 + min(it + kAhead + u, ntiles - 1) * stride);
                 }
                 __syncwarp();
                 if (boff_fill + 8 == 8 * kStages) { boff_fill = 0; eparity ^= 1u; } else boff_fill += 8;
@@ -831,7 +832,7 @@ __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, cons
         } else {
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
-                stage_fill<BITS>(plan, it + kAhead + u < nsteps, it + kAhead + u >= rag_fill, stride, first + (it + kAhead + u) * stride, last, st_fill);
+                stage_fill<BITS>(plan, it + kAhead + u < nsteps, it + kAhead + u >= rag_from, stride, first + (it + kAhead + u) * stride, own_last, st_fill);
                 cp_async_commit();
                 st_fill = (st_fill + kPitch == ring + kStages * kPitch) ? ring : st_fill + kPitch;
             }
