@@ -26,3 +26,25 @@ def test_short_lists_equal_the_batch_calls(dim, n, bits):
         packed, scales = tq.qjl_quantize_batch(cfg, torch.from_numpy(v).cuda(), 5)[:2]
         want = tq.weighted_values(cfg, torch.from_numpy(w).cuda(), packed, scales).cpu().numpy()
         assert np.array_equal(cache.weighted_values(1, w), want)
+
+
+@pytest.mark.parametrize("scores_first", [False, True])
+def test_first_calls_on_a_stream_of_their_own(scores_first):
+    # a non-blocking stream does not wait for what the default stream still has queued
+    rng = np.random.default_rng(3)
+    cfg = tq.TurboQuantConfig(3, 128).with_seed(5)
+    caches = [tq.QuantizedKVCache(cfg, 1, 5) for _ in range(4)]
+    k, v = (rng.standard_normal((700, 128), dtype=np.float32) for _ in range(2))
+    q, w = rng.standard_normal(128, dtype=np.float32), rng.random(700, dtype=np.float32)
+    for c in caches:
+        c.push_batch(0, k, v)
+    want = caches[0].attention_scores(0, q), caches[0].weighted_values(0, w)
+    for c in caches[1:]:
+        torch.cuda._sleep(20_000_000)                       # about 10 ms of work on the default stream
+        for _ in range(2):
+            with torch.cuda.stream(torch.cuda.Stream()):
+                if scores_first:
+                    assert np.array_equal(c.attention_scores(0, q), want[0])
+                assert np.array_equal(c.weighted_values(0, w), want[1])
+        torch.cuda.synchronize()
+        assert np.array_equal(c.weighted_values(0, w), want[1])

@@ -735,13 +735,16 @@ struct tqb_kv_cache {
     unsigned* ticket = nullptr;
     bool map_tried = false;
 
-    bool small_calls(int64_t n) {
+    // `s`: the stream of the call that asks.  The ticket is cleared there and waited for once: a memset on the legacy stream is not
+    // ordered before the work of a non-blocking stream, and the next call may come on another one.
+    bool small_calls(int64_t n, cudaStream_t s) {
         if (n > (int64_t)kMappedFloats - 256) return false;
         if (!map_tried) {
             map_tried = true;
             if (cudaHostAlloc((void**)&mapped, kMappedFloats * sizeof(float), cudaHostAllocMapped) != cudaSuccess ||
                 cudaHostGetDevicePointer((void**)&mapped_dev, mapped, 0) != cudaSuccess ||
-                cudaMalloc((void**)&ticket, 256) != cudaSuccess || cudaMemset(ticket, 0, 256) != cudaSuccess) {
+                cudaMalloc((void**)&ticket, 256) != cudaSuccess || cudaMemsetAsync(ticket, 0, 256, s) != cudaSuccess ||
+                cudaStreamSynchronize(s) != cudaSuccess) {
                 cudaGetLastError();
                 release_small();
             }
@@ -881,7 +884,7 @@ int tqb_kv_cache_attention_scores(tqb_kv_cache* c, int32_t layer, const float* q
     if (!query || !scores) return TQB_ERR_NULL_POINTER;
     cudaStream_t s = as_stream(stream);
     const int d = c->cfg.dim;
-    if (c->small_calls(L.nk)) {
+    if (c->small_calls(L.nk, s)) {
         const int st = launch_scores_query(&c->cfg, c->rbits, query, L.k.packed, L.k.scales, L.k.signs, L.k.rnorms, L.nk, c->mapped_dev, s);
         if (st == TQB_OK) {
             TQB_CUDA(cudaStreamSynchronize(s));
@@ -918,7 +921,7 @@ int tqb_kv_cache_weighted_values(tqb_kv_cache* c, int32_t layer, const float* we
         return TQB_OK;
     }
     if (!weights) return TQB_ERR_NULL_POINTER;
-    if (c->small_calls(n)) {
+    if (c->small_calls(n, s)) {
         TQB_TRY(c->wv_scratch.reserve(tqb_weighted_values_scratch_bytes(d)));
         std::memcpy(c->mapped + 256, weights, (size_t)n * sizeof(float));   // (nothing is in flight: every call ends synchronised)
         const int st = launch_weighted_values_one(&c->cfg, c->mapped_dev + 256, L.v.packed, L.v.scales, n, c->mapped_dev,
