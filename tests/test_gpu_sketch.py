@@ -36,6 +36,27 @@ def test_logit_bias_at_tile_edges(dim, group, q_len, kv_len):
     assert bool(((bias.double() - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("spread", [0.0, 1.0, 2.0, 4.0])
+@pytest.mark.parametrize("dim", [32, 64, 128, 256])
+def test_logit_bias_is_no_less_exact_than_the_sequential_sum(dim, spread):
+    # against 64 bits, beside f32 additions from the first element to the last; log-normal spread over the elements
+    hq, hkv, q_len, kv_len = 8, 2, 37, 300
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    rq = torch.randn((hq, q_len, dim), generator=g, device="cuda") * torch.exp(spread * torch.randn((hq, q_len, dim), generator=g, device="cuda"))
+    signs = torch.randint(0, 256, (hkv, kv_len, dim // 8), generator=g, device="cuda", dtype=torch.uint8)
+    norms = (torch.rand((hkv, kv_len), generator=g, device="cuda") + 0.5).to(torch.float16)
+    bias = torch.empty((hq, q_len, kv_len), device="cuda")
+    assert lib.tqb_qjl_logit_bias(dim, _p(rq), _p(signs), _p(norms), _p(bias), 0, hq, hkv, q_len, kv_len, kv_len, _stream()) == 0
+    pm = (torch.stack([(signs >> b) & 1 for b in range(8)], -1).reshape(hkv, kv_len, dim).float() * 2 - 1).repeat_interleave(hq // hkv, 0)
+    c = (norms.float() * float(np.float32(np.sqrt(np.pi / 2)) / np.sqrt(np.float32(dim)))).repeat_interleave(hq // hkv, 0)[:, None]
+    want = torch.einsum("hid,htd->hit", rq.double(), pm.double()) * c.double()
+    seq = torch.zeros_like(bias)
+    for d in range(dim):
+        seq = seq + rq[:, :, d, None] * pm[:, None, :, d]
+    err, err_seq = ((t.double() - want).norm().item() for t in (bias, seq * c))
+    assert err <= err_seq, (err, err_seq)
+
+
 def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 

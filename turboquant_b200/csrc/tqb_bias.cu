@@ -4,14 +4,16 @@
 //
 // The sum is a dense contraction [g * q_len rows x D] x [D x tokens] with a +-1 operand, so it runs on the tensor cores
 // (mma.sync m16n8k16 bf16, f32 accumulate).  The projected query is split into three bf16 terms, which hold its 24
-// significant bits exactly; +-1 is exact in bf16, so every product is exact and only the f32 accumulation rounds.
+// significant bits exactly; +-1 is exact in bf16, so every product is exact and only the f32 accumulation loses anything.  The tensor
+// cores truncate there, so the leading terms are added up in rounded parts of 16 dims: relative error against 64 bits, normal
+// queries of 128 dims, 4.5e-8 (element by element 2.1e-7, all terms in one accumulator 4.2e-7); wide spreads likewise.
 // A sign bit becomes a bf16 +-1 by one shift and one three-input logic operation per TWO of them (bits p and p + 16 of a
 // sketch word land in the sign positions of the two halves), and the warp keeps the expanded signs of its tokens in
 // registers for all query rows.  What bounds it: the MMAs (768 query-token pairs a clock and SM with three terms) and,
 // at one query token, the output rows.  tcgen05 would have to stage the expanded signs (16 x their stored size) in shared
 // memory for 128 query rows at most; the register-fed MMA never leaves the register file.
 // Measured (32 q / 8 KV heads x 8 sequences, 96 query tokens on 96..384 stored, bf16, mean of four lengths): one thread
-// per token with an f32 FMA per sign 510 us, this kernel 26 us.
+// per token with an f32 FMA per sign 510 us, this kernel 28 us (26 us with one accumulator).
 #include "tqb_common.cuh"
 
 namespace tqb {
@@ -97,19 +99,31 @@ logit_bias_mma_kernel(const float* __restrict__ rq, const uint8_t* __restrict__ 
     float* stage = reinterpret_cast<float*>(s_a + (min(kBiasRows, rows) + 15) / 16 * (KS * 3 * 32)) + warp * 16 * kBiasPitch;
     const int ntok = min(8 * NT, kv_len - tok0);
     for (int mt = 0; mt < tiles; ++mt) {
-        float acc[NT][4];
+        // The tensor cores' accumulation truncates.  So the leading terms (8 bits each) are summed 16 dims at a time into a zero
+        // accumulator, and the parts are added in f32, which rounds; the other two terms, 2^-8 of the sum, stay in one accumulator.
+        float acc[NT][4], small[NT][4];
 #pragma unroll
         for (int i = 0; i < NT; ++i)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][e] = 0.0f;
+            for (int e = 0; e < 4; ++e) acc[i][e] = small[i][e] = 0.0f;
 #pragma unroll
-        for (int ks = 0; ks < KS; ++ks)
+        for (int ks = 0; ks < KS; ++ks) {
+            const uint4* f = s_a + (mt * KS + ks) * 3 * 32 + lane;
+            const uint4 a0 = f[0], a1 = f[32], a2 = f[64];
 #pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                const uint4 a = s_a[((mt * KS + ks) * 3 + t) * 32 + lane];
+            for (int i = 0; i < NT; ++i) {
+                mma_bf16(small[i], a2, b[i][ks][0], b[i][ks][1]);
+                mma_bf16(small[i], a1, b[i][ks][0], b[i][ks][1]);
+                float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                mma_bf16(part, a0, b[i][ks][0], b[i][ks][1]);
 #pragma unroll
-                for (int i = 0; i < NT; ++i) mma_bf16(acc[i], a, b[i][ks][0], b[i][ks][1]);
+                for (int e = 0; e < 4; ++e) acc[i][e] += part[e];
             }
+        }
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][e] += small[i][e];
         // rows n / n + 8 (queries), columns 2j, 2j + 1 (tokens) -> one row of consecutive tokens per store
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
