@@ -1,0 +1,83 @@
+"""The block pool of the cache objects against a counting stand-in for the CUDA allocator (no GPU)."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+PROGRAM = r"""
+#include "tqb_block_pool.h"
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+
+static std::map<char*, size_t> g_live;
+static size_t g_bytes = 0, g_limit = ~(size_t)0, g_calls = 0;
+static char* g_next = (char*)0x100000000;
+extern "C" cudaError_t cudaMalloc(void** p, size_t n) {
+    ++g_calls;
+    if (g_bytes + n > g_limit) return cudaErrorMemoryAllocation;
+    *p = g_next;
+    g_next += (n + 4095) / 4096 * 4096;
+    g_live[(char*)*p] = n;
+    g_bytes += n;
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaFree(void* p) {
+    auto it = g_live.find((char*)p);
+    if (it == g_live.end()) { std::puts("cudaFree of what is not allocated"); std::exit(1); }
+    g_bytes -= it->second;
+    g_live.erase(it);
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaGetLastError() { return cudaSuccess; }
+
+using namespace tqb;
+typedef BlockPool::Block Block;
+#define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); std::exit(1); } } while (0)
+static const size_t MB = 1 << 20;
+static Block take(BlockPool& p, size_t n, int alike = 1, bool use_idle = true) {
+    Block b;
+    CHECK(p.take(n, alike, use_idle, &b) == cudaSuccess);
+    auto it = g_live.upper_bound((char*)b.p);
+    CHECK(it != g_live.begin());
+    --it;
+    CHECK((char*)b.p + n <= it->first + it->second);      // inside an allocation
+    return b;
+}
+"""
+
+RETIRE = """
+int main() {
+    BlockPool p;
+    Block a = take(p, 3 * MB, 4);
+    p.retire(a);                                          // outgrown: queued work may still read it
+    Block b[4];
+    for (auto& x : b) { x = take(p, 3 * MB); CHECK(x.p != a.p); }
+    p.settle();                                           // the device has been waited for
+    CHECK(take(p, 3 * MB).p == a.p);
+    p.release();
+    CHECK(g_bytes == 0);
+}
+"""
+
+
+def run(tmp_path, main):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None or not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime_api.h")):
+        pytest.skip("needs a C++ compiler and the CUDA headers")
+    src, exe = tmp_path / "pool.cpp", tmp_path / "pool"
+    src.write_text(PROGRAM + main)
+    r = subprocess.run([cxx, "-std=c++17", "-Wall", "-Werror", "-I", os.path.join(ROOT, "turboquant_b200", "csrc"), "-isystem",
+                        os.path.join(CUDA, "include"), str(src), "-o", str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
+
+
+def test_a_retired_block_waits_for_the_device(tmp_path):
+    run(tmp_path, RETIRE)

@@ -1,5 +1,7 @@
 """The caches' device memory across growth and reset: blocks that a cache takes again hold what fresh ones would."""
 
+import threading
+
 import pytest
 import torch
 
@@ -48,3 +50,34 @@ def test_reset_gives_large_blocks_back():
         cache.prefill(layer, x, x)
     cache.reset()
     assert free0 - torch.cuda.mem_get_info()[0] <= (512 + 64) << 20
+
+
+@pytest.mark.parametrize("sketch", [False, True])
+def test_growth_beside_a_capture(sketch):
+    # a cache may grow on its stream while another thread has a graph of its own under capture
+    cfg = tq.CacheConfig(bits=3, head_dim=128, num_kv_heads=2, num_layers=1, batch=1, outlier_blocks=0 if sketch else tq.ALL_BLOCKS)
+    cache = (tq.TqCache if sketch else tq.PqoCache)(cfg)
+    rows = torch.randn((1, 2, 200, 128), device="cuda")
+    y, s1, s2, failed = torch.zeros(8, device="cuda"), torch.cuda.Stream(), torch.cuda.Stream(), []
+    torch.cuda.synchronize()
+
+    def fill():
+        try:
+            with torch.cuda.stream(s2):
+                for _ in range(4):
+                    cache.prefill(0, rows, rows, rows[:, :, :1].contiguous()) if sketch else cache.prefill(0, rows, rows)
+        except Exception as e:
+            failed.append(e)
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(s1):
+        graph.capture_begin(capture_error_mode="thread_local")
+        y.add_(1.0)
+        t = threading.Thread(target=fill)
+        t.start()
+        t.join()
+        y.add_(1.0)
+        graph.capture_end()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert not failed and cache.seq_len(0) == 800 and y[0].item() == 2.0

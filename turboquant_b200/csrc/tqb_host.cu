@@ -7,6 +7,7 @@
 #include <new>
 #include <vector>
 
+#include "tqb_block_pool.h"
 #include "tqb_common.cuh"
 #include "tqb_sketch.cuh"
 
@@ -51,93 +52,6 @@ struct DevBuf {
     }
 };
 
-// Blocks of device memory that a cache object gives up (reset, growth) and takes again: cudaMalloc and cudaFree cost
-// 80 to 500 us each and cudaFree waits for the whole device, so a request of 16 steps on 28 layers spent 18 of its 20 ms
-// in them.  Small blocks come from slabs: the layers of a cache grow to the same size one after the other, so the first one
-// asks for all that are as far behind (a new cache's 28 layers of 1,024 tokens stored: 9.1 -> 0.9 ms).
-// The pool belongs to one cache object, keeps at most kKeepBytes idle and is given back with the object or when an allocation
-// fails.  Every idle block is unused: its owner has synchronised the device before it was put here.
-class BlockPool {
-public:
-    static constexpr size_t kKeepBytes = 512u << 20, kSlabBytes = 64u << 20;
-    struct Block {
-        void* p = nullptr;
-        size_t bytes = 0;
-        int slab = -1;
-    };
-
-    // The smallest idle block that fits, unless it is more than twice as large; else a new one, out of a slab of up to
-    // `alike` blocks of the size.  `use_idle` = false while the stream is being captured: whatever cudaMalloc answers there is the answer.
-    cudaError_t take(size_t need, int alike, bool use_idle, Block* out) {
-        if (use_idle && take_idle(need, out)) return cudaSuccess;
-        int count = use_idle && need <= kSlabBytes / 2 ? (int)std::min<size_t>((size_t)alike, kSlabBytes / need) : 1;
-        if (count < 1) count = 1;
-        void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, need * count);
-        if (e == cudaErrorMemoryAllocation && (count > 1 || !idle_.empty())) {
-            cudaGetLastError();
-            trim();
-            count = 1;
-            e = cudaMalloc(&p, need);
-        }
-        if (e != cudaSuccess) return e;
-        const int slab = (int)slabs_.size();
-        slabs_.push_back(Slab{p, count, count});
-        for (int i = 1; i < count; ++i) put(Block{(char*)p + i * need, need, slab});
-        *out = Block{p, need, slab};
-        return cudaSuccess;
-    }
-    void put(const Block& b) {
-        if (!b.p) return;
-        idle_.push_back(b);
-        held_ += b.bytes;
-        --slabs_[b.slab].used;
-        if (held_ > kKeepBytes) trim();
-    }
-    // Frees what no live block shares a slab with.
-    void trim() {
-        for (size_t i = 0; i < slabs_.size(); ++i)
-            if (slabs_[i].used == 0 && slabs_[i].p) {
-                for (size_t k = idle_.size(); k-- > 0;)
-                    if (idle_[k].slab == (int)i) {
-                        held_ -= idle_[k].bytes;
-                        idle_.erase(idle_.begin() + k);
-                    }
-                cudaFree(slabs_[i].p);
-                slabs_[i].p = nullptr;
-            }
-    }
-    // With the object: live blocks too.
-    void release() {
-        for (auto& s : slabs_)
-            if (s.p) cudaFree(s.p);
-        slabs_.clear();
-        idle_.clear();
-        held_ = 0;
-    }
-
-private:
-    struct Slab {
-        void* p;
-        int blocks, used;
-    };
-    std::vector<Block> idle_;
-    std::vector<Slab> slabs_;
-    size_t held_ = 0;
-
-    bool take_idle(size_t need, Block* out) {
-        size_t best = idle_.size();
-        for (size_t i = 0; i < idle_.size(); ++i)
-            if (idle_[i].bytes >= need && idle_[i].bytes / 2 <= need && (best == idle_.size() || idle_[i].bytes < idle_[best].bytes)) best = i;
-        if (best == idle_.size()) return false;
-        *out = idle_[best];
-        held_ -= out->bytes;
-        ++slabs_[out->slab].used;
-        idle_.erase(idle_.begin() + best);
-        return true;
-    }
-};
-
 bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {   // the legacy stream while another one is being captured
@@ -146,8 +60,6 @@ bool capturing(cudaStream_t s) {
     }
     return st != cudaStreamCaptureStatusNone;
 }
-
-size_t align256(size_t n) { return (n + 255) / 256 * 256; }
 
 }  // namespace
 
@@ -271,15 +183,16 @@ struct tqb_pqo_cache {
                 if ((r = cudaMemcpy2DAsync(nl.vs, (size_t)new_cap * nblk * 2, l.vs, (size_t)l.cap * nblk * 2, sw, heads,
                                            cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return r;
             }
-            // the old buffers may still be read by work queued on any stream, and the copies above must have left them
-            return l.ki ? cudaDeviceSynchronize() : cudaSuccess;
+            return l.ki ? cudaStreamSynchronize(s) : cudaSuccess;
         };
         if ((e = fill()) != cudaSuccess) {
-            cudaDeviceSynchronize();   // nothing queued may still write the buffers that are released next
-            free_layer(nl);
+            cudaStreamSynchronize(s);
+            pool.retire(nl.block);   // what is queued may still write it
             return cuda_fail(e);
         }
-        if (l.ki) free_layer(l);
+        // work queued on any stream may still read the old rows: they are not taken again before a reset has waited for the
+        // device (waiting for it here fails while any stream of the process is being captured, and ends that capture)
+        pool.retire(l.block);
         l = nl;
         return TQB_OK;
     }
@@ -660,6 +573,7 @@ int tqb_pqo_cache_reset(tqb_pqo_cache* c) {
     if (!c) return TQB_ERR_NULL_POINTER;
     TQB_CUDA(cudaDeviceSynchronize());
     for (auto& l : c->layers) c->free_layer(l);
+    c->pool.settle();
     return TQB_OK;
 }
 
@@ -1070,6 +984,7 @@ struct tqb_tq_cache {
 
     int sb() const { return base->cfg.head_dim / 8; }
 
+    // (nothing queued uses it any more)
     void free_q(Q& q) {
         base->pool.put(q.block);
         q = Q{};
@@ -1099,14 +1014,14 @@ struct tqb_tq_cache {
                 if ((r = cudaMemcpy2DAsync(n.norms, (size_t)new_cap * 2, q.norms, (size_t)q.cap * 2, (size_t)old_len * 2, heads,
                                            cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return r;
             }
-            return q.signs ? cudaDeviceSynchronize() : cudaSuccess;
+            return q.signs ? cudaStreamSynchronize(s) : cudaSuccess;
         };
         if ((e = fill()) != cudaSuccess) {
-            cudaDeviceSynchronize();
-            free_q(n);
+            cudaStreamSynchronize(s);
+            base->pool.retire(n.block);
             return cuda_fail(e);
         }
-        if (q.signs) free_q(q);
+        base->pool.retire(q.block);
         q = n;
         return TQB_OK;
     }
