@@ -65,6 +65,38 @@ int main() {
 }
 """
 
+BOUND = """
+int main() {
+    BlockPool p;
+    const size_t keep = BlockPool::kKeepBytes;
+    // 28 layers of 40 MB, 1,120 MB: what the pool holds after a reset is the bound's worth of blocks, and the next request
+    // allocates the rest only
+    std::vector<Block> b(28);
+    for (int request = 0; request < 5; ++request) {
+        const size_t before = g_calls;
+        for (auto& x : b) x = take(p, 40 * MB);
+        CHECK(g_calls - before == (request == 0 ? 28u : 28u - keep / (40 * MB)));
+        CHECK(g_bytes == 28 * 40 * MB);
+        for (auto& x : b) p.put(x);
+        p.settle();
+        CHECK(g_bytes <= keep && g_bytes > keep - 40 * MB);
+    }
+    // idle blocks beside a live one come on top of the bound and go with it
+    Block one = take(p, 16 * MB, 4);
+    for (auto& x : b) x = take(p, 40 * MB);
+    for (auto& x : b) p.put(x);
+    CHECK(g_bytes <= keep + 4 * 16 * MB);
+    p.put(one);
+    CHECK(g_bytes <= keep);
+    // an allocation that fails gives back everything unused first
+    g_limit = keep + 8 * MB;
+    take(p, keep);
+    CHECK(g_bytes == keep);
+    p.release();
+    CHECK(g_bytes == 0);
+}
+"""
+
 
 def run(tmp_path, main):
     cxx = shutil.which("g++") or shutil.which("c++")
@@ -81,3 +113,7 @@ def run(tmp_path, main):
 
 def test_a_retired_block_waits_for_the_device(tmp_path):
     run(tmp_path, RETIRE)
+
+
+def test_what_the_pool_holds_is_bounded_and_kept_up_to_the_bound(tmp_path):
+    run(tmp_path, BOUND)

@@ -12,8 +12,9 @@ namespace tqb {
 // 80 to 500 us each and cudaFree waits for the whole device, so a request of 16 steps on 28 layers spent 18 of its 20 ms
 // in them.  Small blocks come from slabs: the layers of a cache grow to the same size one after the other, so the first one
 // asks for all that are as far behind (a new cache's 28 layers of 1,024 tokens stored: 9.1 -> 0.9 ms).
-// The pool belongs to one cache object, keeps at most kKeepBytes idle and is given back with the object or when an allocation
-// fails.  Every idle block is unused: its owner has synchronised the device before it was put here.  A block that a layer outgrows
+// The pool belongs to one cache object and is given back with the object or when an allocation fails.  Beyond kKeepBytes held, wholly
+// unused slabs are freed, the oldest first, until no more than that is held: after a reset the bound is exact.  While the cache
+// is in use, blocks that share a slab with a live one come on top; they go when that one does.  Every idle block is unused: its owner has synchronised the device before it was put here.  A block that a layer outgrows
 // while work may still use it is retired: nothing takes it before settle(), which a reset calls after it has waited for the device.
 class BlockPool {
 public:
@@ -34,7 +35,7 @@ public:
         cudaError_t e = cudaMalloc(&p, need * count);
         if (e == cudaErrorMemoryAllocation && (count > 1 || held_ > 0)) {
             cudaGetLastError();
-            trim();
+            trim(0);
             count = 1;
             e = cudaMalloc(&p, need);
         }
@@ -52,9 +53,10 @@ public:
         idle_.insert(idle_.end(), retired_.begin(), retired_.end());
         retired_.clear();
     }
-    // Frees what no live block shares a slab with (cudaFree waits for work that still uses a retired one).
-    void trim() {
-        for (size_t i = 0; i < slabs_.size(); ++i)
+    // Frees slabs without a live block, the oldest first, until at most `keep` bytes are held (cudaFree waits for work that still uses
+    // a retired block).
+    void trim(size_t keep) {
+        for (size_t i = 0; i < slabs_.size() && held_ > keep; ++i)
             if (slabs_[i].used == 0 && slabs_[i].p) {
                 for (auto* list : {&idle_, &retired_})
                     for (size_t k = list->size(); k-- > 0;)
@@ -90,7 +92,7 @@ private:
         list.push_back(b);
         held_ += b.bytes;
         --slabs_[b.slab].used;
-        if (held_ > kKeepBytes) trim();
+        if (held_ > kKeepBytes) trim(kKeepBytes);
     }
 
     bool take_idle(size_t need, Block* out) {
