@@ -97,6 +97,22 @@ int main() {
 }
 """
 
+RECORDS = """
+int main() {
+    BlockPool p;
+    std::vector<Block> b(28);
+    for (int request = 0; request < 200; ++request) {     // above the bound: slabs come and go with every request
+        for (auto& x : b) x = take(p, (30 + request % 7) * MB, request % 3 + 1);
+        for (auto& x : b) { if (request % 2) p.retire(x); else p.put(x); }
+        p.settle();
+        CHECK(p.slabs() == g_live.size());
+        CHECK(p.slabs() <= 28);
+    }
+    p.release();
+    CHECK(g_bytes == 0 && p.slabs() == 0);
+}
+"""
+
 
 def run(tmp_path, main):
     cxx = shutil.which("g++") or shutil.which("c++")
@@ -117,3 +133,7 @@ def test_a_retired_block_waits_for_the_device(tmp_path):
 
 def test_what_the_pool_holds_is_bounded_and_kept_up_to_the_bound(tmp_path):
     run(tmp_path, BOUND)
+
+
+def test_many_resets_above_the_bound_leave_no_records(tmp_path):
+    run(tmp_path, RECORDS)

@@ -4,6 +4,8 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <list>
+#include <new>
 #include <vector>
 
 namespace tqb {
@@ -17,12 +19,17 @@ namespace tqb {
 // is in use, blocks that share a slab with a live one come on top; they go when that one does.  Every idle block is unused: its owner has synchronised the device before it was put here.  A block that a layer outgrows
 // while work may still use it is retired: nothing takes it before settle(), which a reset calls after it has waited for the device.
 class BlockPool {
+    struct Slab {
+        void* p;
+        int blocks, used;   // used: not idle, not retired
+    };
+
 public:
     static constexpr size_t kKeepBytes = 512u << 20, kSlabBytes = 64u << 20;
     struct Block {
         void* p = nullptr;
         size_t bytes = 0;
-        int slab = -1;
+        Slab* slab = nullptr;
     };
 
     // The smallest idle block that fits, unless it is more than twice as large; else a new one, out of a slab of up to
@@ -40,8 +47,16 @@ public:
             e = cudaMalloc(&p, need);
         }
         if (e != cudaSuccess) return e;
-        const int slab = (int)slabs_.size();
-        slabs_.push_back(Slab{p, count, count});
+        try {   // room for every block in either list: hold() and settle() never allocate
+            idle_.reserve(blocks_ + count);
+            retired_.reserve(blocks_ + count);
+            slabs_.push_back(Slab{p, count, count});
+        } catch (const std::bad_alloc&) {
+            cudaFree(p);
+            return cudaErrorMemoryAllocation;
+        }
+        blocks_ += count;
+        Slab* slab = &slabs_.back();
         for (int i = 1; i < count; ++i) put(Block{(char*)p + i * need, need, slab});
         *out = Block{p, need, slab};
         return cudaSuccess;
@@ -56,42 +71,44 @@ public:
     // Frees slabs without a live block, the oldest first, until at most `keep` bytes are held (cudaFree waits for work that still uses
     // a retired block).
     void trim(size_t keep) {
-        for (size_t i = 0; i < slabs_.size() && held_ > keep; ++i)
-            if (slabs_[i].used == 0 && slabs_[i].p) {
-                for (auto* list : {&idle_, &retired_})
-                    for (size_t k = list->size(); k-- > 0;)
-                        if ((*list)[k].slab == (int)i) {
-                            held_ -= (*list)[k].bytes;
-                            list->erase(list->begin() + k);
-                        }
-                cudaFree(slabs_[i].p);
-                slabs_[i].p = nullptr;
+        for (auto it = slabs_.begin(); it != slabs_.end() && held_ > keep;) {
+            if (it->used > 0) {
+                ++it;
+                continue;
             }
+            for (auto* list : {&idle_, &retired_})
+                for (size_t k = list->size(); k-- > 0;)
+                    if ((*list)[k].slab == &*it) {
+                        held_ -= (*list)[k].bytes;
+                        list->erase(list->begin() + k);
+                    }
+            cudaFree(it->p);
+            blocks_ -= it->blocks;
+            it = slabs_.erase(it);
+        }
     }
+    // Slabs that hold memory (the pool keeps no record of any other).
+    size_t slabs() const { return slabs_.size(); }
     // With the object: live blocks too.
     void release() {
-        for (auto& s : slabs_)
-            if (s.p) cudaFree(s.p);
+        for (auto& s : slabs_) cudaFree(s.p);
         slabs_.clear();
         idle_.clear();
         retired_.clear();
-        held_ = 0;
+        held_ = blocks_ = 0;
     }
 
 private:
-    struct Slab {
-        void* p;
-        int blocks, used;
-    };
     std::vector<Block> idle_, retired_;
-    std::vector<Slab> slabs_;
-    size_t held_ = 0;   // bytes of both lists
+    std::list<Slab> slabs_;   // by age; blocks point into it
+    size_t held_ = 0;         // bytes of both lists
+    size_t blocks_ = 0;       // of all slabs
 
     void hold(const Block& b, std::vector<Block>& list) {
         if (!b.p) return;
         list.push_back(b);
         held_ += b.bytes;
-        --slabs_[b.slab].used;
+        --b.slab->used;
         if (held_ > kKeepBytes) trim(kKeepBytes);
     }
 
@@ -102,7 +119,7 @@ private:
         if (best == idle_.size()) return false;
         *out = idle_[best];
         held_ -= out->bytes;
-        ++slabs_[out->slab].used;
+        ++out->slab->used;
         idle_.erase(idle_.begin() + best);
         return true;
     }
