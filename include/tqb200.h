@@ -409,8 +409,11 @@ int tqb_pqo_cache_dequantize_full(tqb_pqo_cache *c, int32_t layer, void *k_out, 
                                   int32_t host_buffers, tqb_stream_t stream);
 int64_t tqb_pqo_cache_seq_len(const tqb_pqo_cache *c, int32_t layer);
 int64_t tqb_pqo_cache_capacity(const tqb_pqo_cache *c, int32_t layer);
-/* Drops every layer's rows.  Device memory: up to 512 MB of the freed blocks stay with the cache for its next rows and go
- * with tqb_pqo_cache_destroy; the rest is freed. */
+/* Drops every layer's rows.  Device memory: blocks that a layer gives up - here or when it outgrows one - stay with the cache
+ * for its next rows and go with tqb_pqo_cache_destroy, up to 512 MB of them after a reset; the rest is freed.  While the cache
+ * is in use, idle blocks that share an allocation with a block in use come on top.  Layers grow to the same size one after
+ * the other, so a layer's first rows allocate for the layers not yet used too, up to 64 MB, and its later growths for at most as many
+ * unused layers as there are used ones. */
 int tqb_pqo_cache_reset(tqb_pqo_cache *c);
 /* enabled != 0: the decode launches of this cache (tqb_pqo_cache_decode with device buffers, tqb_pqo_cache_attend_partial,
  * tqb_pqo_cache_attend_push) are made with TQB_DECODE_OVERLAP whenever the layer differs from the layer of the

@@ -39,8 +39,8 @@ extern "C" cudaError_t cudaGetLastError() { return cudaSuccess; }
 using namespace tqb;
 typedef BlockPool::Block Block;
 #define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); std::exit(1); } } while (0)
-static const size_t MB = 1 << 20;
-static Block take(BlockPool& p, size_t n, int alike = 1, bool use_idle = true) {
+[[maybe_unused]] static const size_t MB = 1 << 20;
+[[maybe_unused]] static Block take(BlockPool& p, size_t n, int alike = 1, bool use_idle = true) {
     Block b;
     CHECK(p.take(n, alike, use_idle, &b) == cudaSuccess);
     auto it = g_live.upper_bound((char*)b.p);
@@ -113,6 +113,26 @@ int main() {
 }
 """
 
+AHEAD = """
+struct Layer { int64_t cap; };
+int main() {
+    std::vector<Layer> l(80, Layer{0});
+    CHECK(blocks_ahead(l, 0, 100) == 80);                 // a new cache's first prompt
+    l[0].cap = 228;
+    CHECK(blocks_ahead(l, 0, 100) == 79);                 // the second layer's: the first one has its rows
+    CHECK(blocks_ahead(l, l[0].cap, 300) == 2);           // a layer used alone
+    for (int i = 0; i < 28; ++i) l[i].cap = 228;
+    CHECK(blocks_ahead(l, l[0].cap, 300) == 28 + 28);
+    for (auto& x : l) x.cap = 228;
+    l[0].cap = 428;
+    CHECK(blocks_ahead(l, l[1].cap, 300) == 79);
+    std::vector<Layer> one(1, Layer{0});
+    CHECK(blocks_ahead(one, 0, 1) == 1);
+    one[0].cap = 129;
+    CHECK(blocks_ahead(one, 129, 200) == 1);
+}
+"""
+
 
 def run(tmp_path, main):
     cxx = shutil.which("g++") or shutil.which("c++")
@@ -137,3 +157,7 @@ def test_what_the_pool_holds_is_bounded_and_kept_up_to_the_bound(tmp_path):
 
 def test_many_resets_above_the_bound_leave_no_records(tmp_path):
     run(tmp_path, RECORDS)
+
+
+def test_memory_for_layers_that_are_never_used_is_bounded(tmp_path):
+    run(tmp_path, AHEAD)

@@ -81,3 +81,18 @@ def test_growth_beside_a_capture(sketch):
     graph.replay()
     torch.cuda.synchronize()
     assert not failed and cache.seq_len(0) == 800 and y[0].item() == 2.0
+
+
+def test_one_layer_of_many():
+    # the growths of one layer of 80: its first allocation may hold blocks for all, the later ones two each
+    cache = tq.PqoCache(tq.CacheConfig(bits=4, head_dim=128, num_kv_heads=8, num_layers=80, batch=1))
+    x = torch.zeros((1, 8, 64, 128), dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    free0, caps = torch.cuda.mem_get_info()[0], set()
+    for _ in range(200):
+        cache.prefill(79, x, x)
+        caps.add(cache.capacity(79))
+    block = lambda cap: 8 * cap * (2 * 64 + 2 * 8) + 1024
+    bound = 80 * block(min(caps)) + sum(2 * block(c) for c in caps)
+    assert free0 - torch.cuda.mem_get_info()[0] <= bound + len(caps) * (4 << 20)      # 2 MB granules of the driver
+    assert len(caps) > 10

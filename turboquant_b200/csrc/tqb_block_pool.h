@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <cstdint>
 #include <list>
 #include <new>
 #include <vector>
@@ -13,7 +14,7 @@ namespace tqb {
 // Blocks of device memory that a cache object gives up (reset, growth) and takes again: cudaMalloc and cudaFree cost
 // 80 to 500 us each and cudaFree waits for the whole device, so a request of 16 steps on 28 layers spent 18 of its 20 ms
 // in them.  Small blocks come from slabs: the layers of a cache grow to the same size one after the other, so the first one
-// asks for all that are as far behind (a new cache's 28 layers of 1,024 tokens stored: 9.1 -> 0.9 ms).
+// asks for all that are as far behind (`blocks_ahead`; a new cache's 28 layers of 1,024 tokens stored: 9.1 -> 0.9 ms).
 // The pool belongs to one cache object and is given back with the object or when an allocation fails.  Beyond kKeepBytes held, wholly
 // unused slabs are freed, the oldest first, until no more than that is held: after a reset the bound is exact.  While the cache
 // is in use, blocks that share a slab with a live one come on top; they go when that one does.  Every idle block is unused: its owner has synchronised the device before it was put here.  A block that a layer outgrows
@@ -124,6 +125,23 @@ private:
         return true;
     }
 };
+
+// How many blocks of a size a growing layer asks for at once: its own, one for each layer in use that will need the same next, and of
+// the layers never used all at the layer's own first growth (the first prompt of a new cache), later no more than are in use: a
+// program that uses one layer of 80 holds a block more than it needs, not 79.
+template <typename Layers>
+int blocks_ahead(const Layers& layers, int64_t own_cap, int64_t needed) {
+    int behind = 0, used = 0, unused = 0;
+    for (const auto& o : layers) {
+        if (o.cap == 0) {
+            ++unused;
+        } else {
+            ++used;
+            behind += o.cap < needed ? 1 : 0;
+        }
+    }
+    return own_cap == 0 ? behind + unused : behind + std::min(unused, used);
+}
 
 inline size_t align256(size_t n) { return (n + 255) / 256 * 256; }
 

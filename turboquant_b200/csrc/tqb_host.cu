@@ -161,9 +161,7 @@ struct tqb_pqo_cache {
         const size_t sb = (size_t)heads * new_cap * nblk * sizeof(uint16_t);
         const size_t ia = align256(ib), sa = align256(sb);
         cudaError_t e;
-        int alike = 0;   // layers that will ask for the same next
-        for (const auto& o : layers) alike += o.cap < needed ? 1 : 0;
-        if ((e = pool.take(2 * (ia + sa), alike, !capturing(s), &nl.block)) != cudaSuccess) return cuda_fail(e);
+        if ((e = pool.take(2 * (ia + sa), blocks_ahead(layers, l.cap, needed), !capturing(s), &nl.block)) != cudaSuccess) return cuda_fail(e);
         nl.ki = (uint8_t*)nl.block.p;
         nl.vi = nl.ki + ia;
         nl.ks = (uint16_t*)(nl.vi + ia);
@@ -1000,9 +998,7 @@ struct tqb_tq_cache {
         const int heads = base->heads;
         const size_t sa = align256((size_t)heads * new_cap * sb()), bytes = sa + align256((size_t)heads * new_cap * 2);
         cudaError_t e;
-        int alike = 0;
-        for (const auto& o : qjl) alike += o.cap < needed ? 1 : 0;
-        if ((e = base->pool.take(bytes, alike, !capturing(s), &n.block)) != cudaSuccess) return cuda_fail(e);
+        if ((e = base->pool.take(bytes, blocks_ahead(qjl, q.cap, needed), !capturing(s), &n.block)) != cudaSuccess) return cuda_fail(e);
         n.signs = (uint8_t*)n.block.p;
         n.norms = (uint16_t*)(n.signs + sa);
         auto fill = [&]() -> cudaError_t {
