@@ -57,6 +57,29 @@ def test_logit_bias_is_no_less_exact_than_the_sequential_sum(dim, spread):
     assert err <= err_seq, (err, err_seq)
 
 
+@pytest.mark.parametrize("dim", [32, 64, 96, 128, 256])
+def test_logit_bias_of_infinities_and_nan(dim):
+    # a NaN whose bits are all in the low half of the word is none the less one; rows without any are untouched
+    rq = torch.randn((8, 5, dim), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    bits = rq.view(torch.int32)
+    bits[0, 0, 3], bits[0, 1, dim - 1], bits[3, 2, 7] = 0x7F800001, 0x7FC00000, -0x7FFF8000     # NaN; the last one 0x80008000: a denormal
+    bits[4, 4, 0] = 0x7F7F8001                                                                   # the finite end of the range
+    rq[5, 1, 2] = float("inf")
+    rq[6, 2, 5], rq[6, 2, 9] = float("inf"), float("-inf")
+    signs = torch.zeros((2, 40, dim // 8), dtype=torch.uint8, device="cuda")                     # every sign -1
+    norms = torch.ones((2, 40), dtype=torch.float16, device="cuda")
+    bias = torch.empty((8, 5, 40), device="cuda")
+    assert lib.tqb_qjl_logit_bias(dim, _p(rq), _p(signs), _p(norms), _p(bias), 0, 8, 2, 5, 40, 40, _stream()) == 0
+    nan = torch.zeros((8, 5), dtype=torch.bool, device="cuda")
+    nan[0, 0] = nan[0, 1] = nan[6, 2] = True
+    assert torch.equal(bias.isnan(), nan[..., None].expand_as(bias))
+    assert torch.equal(bias[5, 1], torch.full((40,), float("-inf"), device="cuda"))
+    nan[5, 1] = True
+    want = -rq.double().sum(-1) * float(np.float32(np.sqrt(np.pi / 2)) / np.sqrt(np.float32(dim)))
+    err = (bias.double() - want[..., None]).abs() / rq.double().abs().sum(-1)[..., None]
+    assert (err[~nan] < 1e-6).all()
+
+
 def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 

@@ -30,8 +30,9 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint4& a, uint32_t
 }
 
 // x = hi + mid + lo, each a bf16 (the leading 8 bits of what is left, truncated, so nothing overflows): exact for every
-// finite f32 whose low term stays in the normal range.
+// finite f32 whose low term stays in the normal range.  A NaN stays one, whichever of its bits is set.
 __device__ __forceinline__ void split3(float x, uint32_t (&t)[3]) {
+    x = x == x ? x : __uint_as_float(0x7FFFFFFFu);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const uint32_t h = __float_as_uint(x) & 0xFFFF0000u;
