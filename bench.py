@@ -478,7 +478,7 @@ def extra_tq3(tq, w, lib, dev, args, peak):
     return {"workload": "TqCache TQ3 fused decode (in-kernel QJL correction): 4 layers x 64 sequences x 8 kv heads x ctx 8192",
             "value": round(step_bytes / (ms * 1e-3) / 1e9, 1), "unit": "GB/s", "frac_of_hbm_peak": round(step_bytes / (ms * 1e-3) / 1e9 / peak, 4),
             "us_per_layer": round(ms * 1e3 / L, 1), "algorithmic_bytes_per_token_head": bpt,
-            "note": "per layer: block quantize K and V, dequantize K, residual sketch, query projection, then one attention launch"}
+            "note": "per layer: one launch that quantizes K and V, sketches the residual and projects the queries, then one attention launch"}
 
 
 def extra_config3(tq, w, lib, dev, args, peak):

@@ -441,8 +441,8 @@ __device__ __forceinline__ void stage_fill(FillPlan& f, bool issue, bool ragged,
 // (tq_attention_kernel.cu:197-231), norm_t * sqrt(pi/2) / sqrt(128) * sum_d rq[h, d] * (+-1 by the token's sign
 // sketch), computed on the integer tensor-core path: the 128 sign bits of a token enter as 0 / 1 bytes (one shift and
 // one AND per four of them), the projected query rq as a 20-bit integer in three base-256 digits, and
-// sum rq (2 bit - 1) = 2 sum rq bit - sum rq.  The sketch words and norms are fetched straight from global memory one
-// step ahead of their use (16 + 2 bytes per token; they are not staged).
+// sum rq (2 bit - 1) = 2 sum rq bit - sum rq.  The sketch words and norms are fetched straight from global memory two
+// groups of 16 tokens ahead of their use (16 + 2 bytes per token; they are not staged).
 template <typename QT, int BITS, bool NSPLIT, bool TMA, bool QJL = false>
 __global__ void __launch_bounds__(kThreads, 4) decode_mma_kernel(MmaArgs a, const __grid_constant__ TmaMaps maps,
                                                                  const __grid_constant__ Codebook app_cb) {

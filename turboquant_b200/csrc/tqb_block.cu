@@ -356,7 +356,7 @@ block_quantize_pqo_staged_kernel(QuantArgs a, Codebook cb) {
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncwarp();
         float v[32];
-        unpack32<float>(mine + buf * (32 * kPitch), v);
+        unpack32(mine + buf * (32 * kPitch), v);
         __syncwarp();   // the tile is free for the fetch after next
         uint32_t w[4];
         const float scale = pqo_quantize_values<BITS, NORMAL>(v, cb, a.outer_centroid, w, lut);

@@ -15,7 +15,7 @@
 //                        dequantized with its scale to f16 (MN-major B operand in shared memory), N = 128 dims, one
 //                        128 x 128 f32 accumulator per softmax group G.
 // Two softmax groups of four warps each: group G takes tile 2 j + G of every step (columns 64 G .. 64 G + 63 of the
-// step's scores) with its own running (max, sum), P buffer and O accumulator - two independent online softmaxes over
+// step's scores) with its own running (max, sum) and O accumulator - two independent online softmaxes over
 // the even and the odd tiles, merged once at the end like two split-K partitions.  Thread r of a group owns query
 // row r = tensor-memory lane r, so the online softmax needs no shuffles; the output is rotated back in registers
 // (one 32-point butterfly per block) at the end.
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
                         umma_f16_ts(tmemO + G * kD, tmemS + (j & 1) * 2 * kTile + G * kTile + kk * 8, vv + (uint64_t)((kk * 2048) >> 4),
                                     idescO, (j | kk) ? 1u : 0u);
                     }
-                    umma_commit(bar + kVEmpty + 8 * G);      // frees this V stage and P buffer when the MMAs issued so far are done
+                    umma_commit(bar + kVEmpty + 8 * G);      // frees this V stage and the group's P when the MMAs issued so far are done
                 }
             }
             if (ok) umma_commit(bar + kOFull);           // everything issued so far has completed when this arrives
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
     } else {
         // ================= softmax, correction, epilogue: two groups of four warps, thread = query row =================
         // Group G takes tile 2 j + G of every step j (columns 64 G .. 64 G + 63 of the step's scores), with its own
-        // running (max, sum), P buffer and O accumulator: two independent online softmaxes over the even and the odd
+        // running (max, sum) and O accumulator: two independent online softmaxes over the even and the odd
         // tiles, merged once at the end like two split-K partitions.
         const int G = warp >> 2;
         const int r = tid & 127;
@@ -498,8 +498,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_umma_kernel(ChunkArgs a) {
             }
             const float2 lt = halves(add2(add2(ls[0], ls[1]), add2(ls[2], ls[3])));
             l_run = l_run * resc + (lt.x + lt.y);
-            // The group's P V product of the previous step must be done: it wrote the O accumulator rescaled here (and,
-            // with P in shared memory, read the P buffer written below).  The wait is also the flow control of the
+            // The group's P V product of the previous step must be done: it wrote the O accumulator rescaled here.  The wait is also the flow control of the
             // p_full barrier: without it a group could arrive for steps j and j + 1 before the issuing thread has looked
             // at step j, and a parity wait cannot tell a phase from the one two later (seen as bounded waits running
             // out when it was made conditional on a rescale).

@@ -6,8 +6,6 @@
 #include "tqb_common.cuh"
 #include "tqb_f32x2.cuh"
 
-#include <type_traits>
-
 namespace tqb {
 
 template <typename T>
@@ -48,26 +46,15 @@ __device__ __forceinline__ void load32<__half>(const __half* p, float (&v)[32]) 
     }
 }
 
-// 32 values from 16-byte pieces in shared memory
-template <typename T>
+// 32 f32 values from 16-byte pieces in shared memory
 __device__ __forceinline__ void unpack32(const unsigned char* p, float (&v)[32]) {
-    constexpr int kPer = 16 / (int)sizeof(T);
 #pragma unroll
-    for (int k = 0; k < 32 / kPer; ++k) {
-        const uint4 r = *reinterpret_cast<const uint4*>(p + 16 * k);
-        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if constexpr (sizeof(T) == 4) v[4 * k + i] = __uint_as_float(w[i]);
-            else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-                v[8 * k + 2 * i] = __uint_as_float(w[i] << 16);
-                v[8 * k + 2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-            } else {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-                v[8 * k + 2 * i] = f.x;
-                v[8 * k + 2 * i + 1] = f.y;
-            }
-        }
+    for (int k = 0; k < 8; ++k) {
+        const float4 r = *reinterpret_cast<const float4*>(p + 16 * k);
+        v[4 * k] = r.x;
+        v[4 * k + 1] = r.y;
+        v[4 * k + 2] = r.z;
+        v[4 * k + 3] = r.w;
     }
 }
 
@@ -180,7 +167,9 @@ __device__ __forceinline__ float pqo_quantize_values(const float (&v)[32], const
             const F2 rot = mul2(p[i], signed2(pp, pn, np, nn, i));
             const F2 q = mul2(rot, r2);
             const F2 rem = fma2(q, ns2, rot);
-            const float2 t = halves(fma2(rem, r2, q));           // == rot / scale, correctly rounded
+            // rot / scale, correctly rounded: Markstein's correction of a quotient by its remainder (IBM J. Res. Dev. 34, 1990),
+            // r being the correctly rounded reciprocal
+            const float2 t = halves(fma2(rem, r2, q));
             if (lut != nullptr) {
                 const float2 y = halves(fma2(q, f2(kCellScale), f2(kCellHalf + kMagic)));   // k in the low mantissa bits
                 // byte offset of [k >> 8][lane]: a cell row is 256 bytes
