@@ -57,6 +57,32 @@ def test_logit_bias_is_no_less_exact_than_the_sequential_sum(dim, spread):
     assert err <= err_seq, (err, err_seq)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dim", [32, 64, 128, 256])
+@pytest.mark.parametrize("group,q_len,kv_len", [(1, 1, 1), (1, 1, 128), (1, 1, 1000), (2, 1, 129), (1, 2, 300), (3, 1, 257)])
+def test_logit_bias_of_few_rows(dim, group, q_len, kv_len, dtype):
+    # one row, and two from 128 dims on, are summed from the first element to the last; beyond that on the tensor cores
+    hkv, stride, rows = 3, kv_len + 1, group * q_len
+    g = torch.Generator(device="cuda").manual_seed(dim + kv_len)
+    rq = torch.randn((hkv * group, q_len, dim), generator=g, device="cuda")
+    signs = torch.randint(0, 256, (hkv, stride, dim // 8), generator=g, device="cuda", dtype=torch.uint8)
+    norms = torch.rand((hkv, stride), generator=g, device="cuda").to(torch.float16)
+    bias = torch.empty((hkv * group, q_len, kv_len), device="cuda", dtype=dtype)
+    assert lib.tqb_qjl_logit_bias(dim, _p(rq), _p(signs), _p(norms), _p(bias), 0 if dtype == torch.float32 else 2, hkv * group, hkv, q_len, kv_len,
+                                  stride, _stream()) == 0
+    pm = (torch.stack([(signs >> b) & 1 for b in range(8)], -1).reshape(hkv, stride, dim)[:, :kv_len].float() * 2 - 1).repeat_interleave(group, 0)
+    factor = np.float32(np.sqrt(np.pi / 2)) / np.sqrt(np.float32(dim))
+    c = (norms[:, :kv_len].float() * float(factor)).repeat_interleave(group, 0)[:, None]
+    seq = torch.zeros((hkv * group, q_len, kv_len), device="cuda")
+    for d in range(dim):
+        seq = seq + rq[:, :, d, None] * pm[:, None, :, d]
+    if rows == 1 or (rows == 2 and dim >= 128):
+        assert torch.equal(bias, (seq * c).to(dtype))
+    else:   # the additions of both sums: dim roundings of 2^-24 each, and the output's own
+        bound = rq.double().abs().sum(-1)[..., None] * c.double() * dim * 2.0 ** -23 + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23) * (seq * c).abs()
+        assert ((bias.double() - (seq * c).double()).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("dim", [32, 64, 96, 128, 256])
 def test_logit_bias_of_infinities_and_nan(dim):
     # a NaN whose bits are all in the low half of the word is none the less one; rows without any are untouched
