@@ -466,10 +466,12 @@ block_dequantize_lane_kernel(DequantArgs a, Codebook cb) {
     __shared__ __align__(2048) unsigned char s_tab[2 * kTabB];
     __shared__ __align__(16) unsigned char s_stage[kThreads * kPitch];
     const int lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < 2 * kCodes * 32; i += kThreads) {
-        const int code = (i >> 5) & (kCodes - 1);
+#pragma unroll
+    for (int k = 0; k < kCodes * 32 / kThreads; ++k) {
+        const int i = (int)threadIdx.x + k * kThreads, code = i >> 5;
         const float v = cb.c[code < cb.n ? code : cb.n - 1] * a.sign_mag;
-        reinterpret_cast<float*>(s_tab)[i] = i < kCodes * 32 ? v : -v;
+        reinterpret_cast<float*>(s_tab)[i] = v;
+        reinterpret_cast<float*>(s_tab)[i + kCodes * 32] = -v;
     }
     __syncthreads();
     const uint32_t tab = (uint32_t)__cvta_generic_to_shared(s_tab) + lane * 4;

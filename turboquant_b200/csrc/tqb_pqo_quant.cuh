@@ -81,21 +81,23 @@ constexpr uint32_t kSignMask = 0xB1A6D4B2u;   // bit j set <=> sign j is -1 (pre
 // boundaries below t.  .x = that boundary (3e38 when the cell has none), .y = the number of boundaries under the cell.
 // Stored [cell][lane]: the 32 look-ups of a warp instruction touch 32 different bank pairs (256 unreplicated cells met
 // ~6 wavefronts a look-up).  |t| <= outer centroid (2.1573) < 2.2 by construction of the MaxNorm scale, so k stays inside.
-constexpr int kCells = 32;
+constexpr int kCells = 32, kMaxCellBounds = 7;   // codebooks of up to eight entries
 constexpr float kCellScale = 1856.0f;
 constexpr float kCellHalf = 4096.0f;   // an integer, so that kCellHalf + 1.5 * 2^23 is exact
 constexpr float kCellSlop = 1e-3f;
 __device__ __forceinline__ void build_cell_table(const Codebook& cb, int n_bnd, float2* lut, int tid, int nthreads) {
+    // (no division and no loop of unknown length: a launch of a few blocks is mostly this table, 3.0 -> 2.4 us for one row)
+    constexpr float kStep = 256.0f / kCellScale, kLo = (-0.5f - kCellHalf) / kCellScale - kCellSlop, kHi = (255.5f - kCellHalf) / kCellScale + kCellSlop;
+#pragma unroll 4
     for (int i = tid; i < kCells * 32; i += nthreads) {
-        const int c = i >> 5;
-        const float lo = (256.0f * c - 0.5f - kCellHalf) / kCellScale - kCellSlop;
-        const float hi = (256.0f * c + 255.5f - kCellHalf) / kCellScale + kCellSlop;
+        const float at = kStep * (float)(i >> 5), lo = at + kLo, hi = at + kHi;
         float bnd = 3.0e38f;
         float below = 0.0f;
-        for (int k = 0; k < n_bnd; ++k) {
-            const float b = cb.b[k];
-            if (b < lo) below += 1.0f;
-            else if (b <= hi) bnd = b;
+#pragma unroll
+        for (int k = 0; k < kMaxCellBounds; ++k) {
+            const float b = k < n_bnd ? cb.b[k] : 3.0e38f;
+            below += b < lo ? 1.0f : 0.0f;
+            bnd = (b >= lo && b <= hi) ? b : bnd;
         }
         lut[i] = make_float2(bnd, below);
     }
