@@ -613,19 +613,11 @@ scores_query_kernel(const __grid_constant__ QueryArg query, const uint32_t* __re
 constexpr int kWvBlocks = 296;  // two CTAs per SM
 constexpr long long kListMin = 4096;   // shorter lists stay on the warp-per-key kernels (no table build)
 
-// 256 threads
+// 256 threads; v: this warp's sum over its partials
 template <int EPL>
-__device__ __forceinline__ void weighted_values_final(const float* partial, int nparts, float* __restrict__ out, uint64_t seed,
-                                                      float inv_sqrt_d, float (*s_part)[32 * EPL]) {
-    constexpr int D = 32 * EPL;
+__device__ __forceinline__ void weighted_values_final(float (&v)[EPL], float* __restrict__ out, uint64_t seed, float inv_sqrt_d,
+                                                      float (*s_part)[32 * EPL]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float v[EPL];
-#pragma unroll
-    for (int k = 0; k < EPL; ++k) v[k] = 0.0f;
-    for (int p = warp; p < nparts; p += 8) {
-#pragma unroll
-        for (int k = 0; k < EPL; ++k) v[k] += __ldcg(partial + (size_t)p * D + lane + 32 * k);
-    }
 #pragma unroll
     for (int k = 0; k < EPL; ++k) s_part[warp][lane + 32 * k] = v[k];
     __syncthreads();
@@ -642,17 +634,30 @@ __device__ __forceinline__ void weighted_values_final(const float* partial, int 
     for (int k = 0; k < EPL; ++k) out[lane + 32 * k] = (v[k] * inv_sqrt_d) * sign_of(seed, lane + 32 * k);
 }
 
+// Plain read-only loads, of which the compiler keeps several rows in flight (past L1, as the single launch below has to read them,
+// or four rows at a time: 32 dims, 4,095 values 5.0 -> 6.6 us)
 template <int EPL>
 __global__ void __launch_bounds__(256)
 weighted_values_final_kernel(const float* __restrict__ partial, int nparts, float* __restrict__ out, uint64_t seed,
                              float inv_sqrt_d) {
-    __shared__ float s_part[8][32 * EPL];
-    weighted_values_final<EPL>(partial, nparts, out, seed, inv_sqrt_d, s_part);
+    constexpr int D = 32 * EPL;
+    __shared__ float s_part[8][D];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float v[EPL];
+#pragma unroll
+    for (int k = 0; k < EPL; ++k) v[k] = 0.0f;
+    for (int p = warp; p < nparts; p += 8) {
+#pragma unroll
+        for (int k = 0; k < EPL; ++k) v[k] += partial[(size_t)p * D + lane + 32 * k];
+    }
+    weighted_values_final<EPL>(v, out, seed, inv_sqrt_d, s_part);
 }
 
 // weighted_values (src/attention.rs:371-408), accumulated in the rotated domain:
 // sum_t w_t s_t sigma .* H(c_t)/sqrt(d) = sigma .* H(sum_t w_t s_t c_t)/sqrt(d).
-template <int EPL>
+// ONE: the CTA that arrives last adds the partials up, no second launch (a variant of its own: the two-launch one stays as lean as it was,
+// 256 dims, 1,000 values 7.9 -> 7.1 us).
+template <int EPL, bool ONE>
 __global__ void weighted_values_partial_kernel(const float* __restrict__ w, const uint8_t* __restrict__ packed,
                                                const uint16_t* __restrict__ scales, long long n,
                                                float* __restrict__ partial, Codebook cb, int bits, int pb, unsigned* ticket,
@@ -693,17 +698,23 @@ __global__ void weighted_values_partial_kernel(const float* __restrict__ w, cons
         for (int ww = 0; ww < warps; ++ww) s += s_acc[ww][e];
         partial[(size_t)blockIdx.x * D + e] = s;
     }
-    if (ticket == nullptr) return;
-    // the CTA that arrives last adds the partials up: no second launch
-    __shared__ int s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1 : 0;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    weighted_values_final<EPL>(partial, (int)gridDim.x, out, seed, inv_sqrt_d, s_acc);
-    if (threadIdx.x == 0) *ticket = 0u;   // ready for the next call
+    if constexpr (ONE) {
+        __shared__ int s_last;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1 : 0;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+#pragma unroll
+        for (int k = 0; k < EPL; ++k) acc[k] = 0.0f;
+        for (int p = warp; p < (int)gridDim.x; p += 8) {   // written by the other CTAs of this launch: past L1
+#pragma unroll
+            for (int k = 0; k < EPL; ++k) acc[k] += __ldcg(partial + (size_t)p * D + lane + 32 * k);
+        }
+        weighted_values_final<EPL>(acc, out, seed, inv_sqrt_d, s_acc);
+        if (threadIdx.x == 0) *ticket = 0u;   // ready for the next call
+    }
 }
 
 // ---- long key / value lists: one lane per 32 consecutive elements ---------------------------------------
@@ -1271,7 +1282,7 @@ int tqb_weighted_values(const tqb_config* cfg, const float* w, const uint8_t* pa
         return check_launch(s);
     }
     TQB_DISPATCH_EPL(cfg->dim, {
-        weighted_values_partial_kernel<EPL><<<nparts, 256, 0, s>>>(w, packed, scales, n, partial, cb, polar.bits, pb, nullptr, nullptr, 0, 0.0f);
+        weighted_values_partial_kernel<EPL, false><<<nparts, 256, 0, s>>>(w, packed, scales, n, partial, cb, polar.bits, pb, nullptr, nullptr, 0, 0.0f);
         weighted_values_final_kernel<EPL><<<1, 256, 0, s>>>(partial, nparts, out, cfg->rotation_seed, host_inv_sqrt(cfg->dim));
     });
     return check_launch(s);
@@ -1302,7 +1313,7 @@ int tqb::launch_weighted_values_one(const tqb_config* cfg, const float* w, const
     if (n >= kListMin || dim > 256 || !whole_codebook(bits, dim, cb)) return TQB_ERR_UNSUPPORTED;
     int nparts = (int)((n + 7) / 8);
     if (nparts > kWvBlocks) nparts = kWvBlocks;
-    TQB_DISPATCH_EPL(dim, (weighted_values_partial_kernel<EPL><<<nparts, 256, 0, s>>>(
+    TQB_DISPATCH_EPL(dim, (weighted_values_partial_kernel<EPL, true><<<nparts, 256, 0, s>>>(
         w, packed, scales, n, partial, cb, bits, (int)tqb_packed_bytes(bits, dim), ticket, out, cfg->rotation_seed, host_inv_sqrt(dim))));
     return check_launch(s);
 }
