@@ -149,7 +149,9 @@ int tqb_qjl_rademacher_bits(int32_t dim, uint64_t qjl_seed, uint32_t *host_out);
 int tqb_qjl_quantize_batch(const tqb_config *cfg, const uint32_t *rbits, const float *x, int64_t n,
                            uint8_t *packed, uint16_t *scales, uint8_t *signs, uint16_t *rnorms,
                            tqb_stream_t stream);
-/* precompute_query_projections (src/qjl.rs:488-492) for nq queries: rq [nq, dim]. */
+/* precompute_query_projections (src/qjl.rs:488-492) for nq queries: rq [nq, dim].  Added from the first element to the last,
+ * whatever nq is.  (The TQ cache's own projections of 16-bit queries are added on the tensor cores from 2,048 queries a call on,
+ * head_dim 64 and more: the same to f32 rounding, not bit for bit those of a smaller call.) */
 int tqb_qjl_query_projections(int32_t dim, const uint32_t *rbits, const float *q, int64_t nq, float *rq,
                               tqb_stream_t stream);
 /* QuantizedKVCache::attention_scores (src/attention.rs:319-353): raw, unscaled,
@@ -472,7 +474,9 @@ int tqb_residual_sketch(int32_t dim, const uint32_t *rbits, const void *original
                         int64_t rows_per_group, int64_t out_group_stride, int64_t out_row_offset,
                         tqb_stream_t stream);
 /* compute_logit_bias (src/cache/tq.rs:185-253): bias[h, i, t] = (sum_d rq[h, i, d] * sign_td) * norm_t *
- * sqrt(pi/2) / sqrt(head_dim).  rq: device [num_q_heads, q_len, head_dim] f32 (tqb_qjl_query_projections);
+ * sqrt(pi/2) / sqrt(head_dim).  The order of the f32 additions depends on the number of query rows of a KV head: one row
+ * (two from 128 dims on) from the first element to the last, more in parts of 16 on the tensor cores; the error against 64 bits is
+ * that of the sequential sum or less.  rq: device [num_q_heads, q_len, head_dim] f32 (tqb_qjl_query_projections);
  * signs [num_kv_heads, kv_stride, head_dim/8]; norms [num_kv_heads, kv_stride];
  * bias: device [num_q_heads, q_len, kv_len] of bias_dtype. */
 int tqb_qjl_logit_bias(int32_t head_dim, const float *rq, const uint8_t *signs, const uint16_t *norms, void *bias,

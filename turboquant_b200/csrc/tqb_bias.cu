@@ -9,11 +9,12 @@
 // queries of 128 dims, 4.5e-8 (element by element 2.1e-7, all terms in one accumulator 4.2e-7); wide spreads likewise.
 // A sign bit becomes a bf16 +-1 by one shift and one three-input logic operation per TWO of them (bits p and p + 16 of a
 // sketch word land in the sign positions of the two halves), and the warp keeps the expanded signs of its tokens in
-// registers for all query rows.  What bounds it: the MMAs (768 query-token pairs a clock and SM with three terms) and,
-// at one query token, the output rows.  tcgen05 would have to stage the expanded signs (16 x their stored size) in shared
+// registers for all query rows.  What bounds it: the latency of the prologue's loads and of few, short row tiles (stalls on
+// loads 4.4 to 5.4 per issue, tensor pipe 19 to 26 % at 96 query tokens on 192 and 384).  tcgen05 would have to stage the expanded signs (16 x their stored size) in shared
 // memory for 128 query rows at most; the register-fed MMA never leaves the register file.
 // Measured (32 q / 8 KV heads x 8 sequences, 96 query tokens on 96..384 stored, bf16, mean of four lengths): one thread
-// per token with an f32 FMA per sign 510 us, this kernel 28 us (26 us with one accumulator).
+// per token with an f32 FMA per sign 510 us, this kernel 32.8 us launch after launch (30.6 us with one
+// accumulator).
 #include "tqb_common.cuh"
 
 namespace tqb {
